@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <array>
 #include <map>
+#include <unordered_map>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -69,6 +70,7 @@ void free_all(asd_handle* h) {
     }
     if (h->h_err) cudaFreeHost(h->h_err);
     F(h->d_err); F(h->d_aos); F(h->d_check); F(h->d_rep_of_tile); F(h->d_ttm); F(h->d_q4ptr); F(h->d_q4jkl);
+    F(h->pat.row); F(h->pat.ent);
     F(h->sell.lwords); F(h->sell.span_ptr); F(h->sell.spans);
     F(h->sell.slice_ptr); F(h->sell.a); F(h->sell.b); F(h->sell.c); F(h->sell.col); F(h->sell.val);
     F(h->sell.typed); F(h->sell.tab_f); F(h->sell.tab_d);
@@ -140,9 +142,66 @@ struct TensorTable {
     }
 };
 
+// Row patterns of a typed matrix (PatDev): every row's sequence of (column - row, tensor id).
+// Kept when it compresses the matrix: at most 65,536 patterns whose padded table is no more than
+// a quarter of the entries, and rows of nearly equal length (the pattern rows are padded to the
+// longest, the SELL slices only to their own longest).
+void build_patterns(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vector<uint32_t>& adj,
+                    const std::vector<uint32_t>& id, uint32_t sell_entries) {
+    const uint32_t n = h->n;
+    uint32_t W = 0;
+    for (uint32_t i = 0; i < n; i++) W = std::max(W, xadj[i + 1] - xadj[i]);
+    if (W == 0 || (uint64_t)W * n > (uint64_t)sell_entries + sell_entries / 4) return;
+    std::vector<int2> ent;                            // [pattern][W]
+    std::vector<uint32_t> plen;                       // its entries before the padding
+    std::vector<uint16_t> row(n);
+    std::unordered_multimap<uint64_t, uint32_t> seen;  // hash of a pattern -> its number
+    std::vector<int2> cur(W);
+    const size_t most = std::min<size_t>(65536, adj.size() / (4 * (size_t)W));
+    for (uint32_t i = 0; i < n; i++) {
+        const uint32_t len = xadj[i + 1] - xadj[i];
+        const uint32_t* col = adj.data() + xadj[i];
+        const uint32_t* typ = id.data() + xadj[i];
+        auto same = [&](uint32_t p) {
+            const int2* e = ent.data() + (size_t)p * W;
+            for (uint32_t k = 0; k < len; k++)
+                if ((uint32_t)e[k].x != col[k] - i || (uint32_t)e[k].y != typ[k]) return false;
+            return plen[p] == len;
+        };
+        // a lattice repeats the pattern of one of the last rows nearly always
+        uint32_t p = ~0u;
+        for (uint32_t back = 1; back <= 4 && back <= i && p == ~0u; back++)
+            if (same(row[i - back])) p = row[i - back];
+        if (p == ~0u) {
+            for (uint32_t k = 0; k < W; k++)
+                cur[k] = k < len ? make_int2((int)(col[k] - i), (int)typ[k]) : make_int2(0, 0);
+            uint64_t hash = 0xcbf29ce484222325ull;     // FNV-1a over the words
+            for (const int2& v : cur) {
+                hash = (hash ^ (uint32_t)v.x) * 0x100000001b3ull;
+                hash = (hash ^ (uint32_t)v.y) * 0x100000001b3ull;
+            }
+            const auto range = seen.equal_range(hash);
+            for (auto it = range.first; it != range.second && p == ~0u; ++it)
+                if (same(it->second)) p = it->second;
+            if (p == ~0u) {
+                p = (uint32_t)(ent.size() / W);
+                if (p >= most) return;
+                ent.insert(ent.end(), cur.begin(), cur.end());
+                plen.push_back(len);
+                seen.emplace(hash, p);
+            }
+        }
+        row[i] = (uint16_t)p;
+    }
+    h->pat.W = W;
+    h->pat.npat = (uint32_t)(ent.size() / W);
+    h->pat.row = dupload(row.data(), row.size());
+    h->pat.ent = dupload(ent.data(), ent.size());
+}
+
 // CSR (all replicas concatenated) -> SELL-32 device layout.
 void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vector<uint32_t>& adj,
-                const std::vector<double>& val9) {
+                const double* val9) {
     const uint32_t n = h->n;
     const bool full = h->full != 0;
     const bool zz_yy = (h->p.flags & ASD_FLAG_GPU_DZZ_FROM_DYY) != 0;
@@ -189,6 +248,7 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
                     }
             }
             h->sell.typed = dupload(w.data(), w.size());
+            build_patterns(h, xadj, adj, id, E);
             h->h_words = std::move(w);
             h->sell.colbits = 32 - tb;
             h->sell.ntypes = tt.size();
@@ -261,16 +321,25 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
 // summed.  Builds nothing (returns false) for other matrices, several replicas or the streamed
 // layout.
 bool build_dia_alt(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vector<uint32_t>& adj,
-                   const std::vector<double>& val9) {
+                   const double* val9) {
     if (h->nrep != 1 || (h->p.flags & ASD_FLAG_STREAMED_EXCHANGE) || h->p.precision == ASD_FP64_PLAIN) return false;
     const uint32_t n = h->n;
     constexpr uint32_t MAXD = 32;
     std::map<int64_t, uint32_t> offs;
+    // the offset last seen at each position of a row: a lattice repeats it nearly always
+    std::array<int64_t, 64> lo;
+    std::array<uint32_t, 64> ld{};
+    lo.fill(INT64_MAX);
     for (uint32_t i = 0; i < n; i++)
         for (uint32_t k = xadj[i]; k < xadj[i + 1]; k++) {
-            offs.emplace((int64_t)adj[k] - (int64_t)i, 0u);
+            const int64_t o = (int64_t)adj[k] - (int64_t)i;
+            int64_t& last = lo[(k - xadj[i]) & 63u];
+            if (o == last) continue;
+            last = o;
+            offs.emplace(o, 0u);
             if (offs.size() > MAXD) return false;
         }
+    lo.fill(INT64_MAX);
     if (offs.empty()) return false;
     std::vector<int32_t> off;
     for (auto& kv : offs) { kv.second = (uint32_t)off.size(); off.push_back((int32_t)kv.first); }
@@ -285,7 +354,10 @@ bool build_dia_alt(asd_handle* h, const std::vector<uint32_t>& xadj, const std::
     for (uint32_t i = 0; i < n; i++) {
         used.fill(false);
         for (uint32_t k = xadj[i]; k < xadj[i + 1]; k++) {
-            const uint32_t d = offs[(int64_t)adj[k] - (int64_t)i];
+            const int64_t o = (int64_t)adj[k] - (int64_t)i;
+            const uint32_t slot = (k - xadj[i]) & 63u;
+            if (o != lo[slot]) { lo[slot] = o; ld[slot] = offs[o]; }
+            const uint32_t d = ld[slot];
             if (!used[d]) { loc[d].fill(0.0); used[d] = true; }
             for (int q = 0; q < nc; q++) {
                 int src = full ? q : qmap[q];
@@ -514,12 +586,17 @@ bool build_spin_stage(asd_handle* h, int B) {
 }
 
 // Launch shape of the fused stage kernel: block size and the staging mode of typed SELL
-// words (0 none, 1 words, 2 words and neighbour spins).
+// words (0 none, 1 words, 2 words and neighbour spins, STAGE_PATTERN row patterns instead of the
+// words where the matrix has them, else 1).
 void configure_stage(asd_handle* h, int B, int mode) {
     h->block = B;
     h->sell.stage = 0;
     h->sell.stage_words = 0;
     if (mode == 0 || !h->sell.typed || h->dexch != ASD_EXCH_CSR) return;
+    if (mode == (int)STAGE_PATTERN) {
+        if (h->pat.W) { h->sell.stage = STAGE_PATTERN; return; }
+        mode = 1;
+    }
     const size_t rb = h->p.precision == ASD_FP32 ? 4 : 8;
     const size_t tab = ((rb * (h->full ? 12 : 4) * h->sell.ntypes) + 15) & ~(size_t)15;
     const uint32_t w = stage_capacity(h, B);
@@ -536,7 +613,7 @@ void configure_stage(asd_handle* h, int B, int mode) {
 // for every block size in {64, 128, 256} with and without staging, keep the fastest.
 void autotune(asd_handle* h) {
     struct Cand { uint32_t layout; int B; int mode; };
-    static const char* names[3] = {"direct", "words", "words+spins"};
+    static const char* names[4] = {"direct", "words", "words+spins", "pattern"};
     std::vector<Cand> cs;
     // DIA input also exists as SELL-32, and a CSR matrix on few diagonals as DIA: both device
     // layouts are candidates
@@ -547,6 +624,7 @@ void autotune(asd_handle* h) {
         for (int B : {64, 128, 256}) {
             cs.push_back({lay, B, 0});
             if (h->sell.typed && lay == ASD_EXCH_CSR) { cs.push_back({lay, B, 1}); cs.push_back({lay, B, 2}); }
+            if (h->pat.W && lay == ASD_EXCH_CSR) cs.push_back({lay, B, (int)STAGE_PATTERN});
         }
     double best = 1e300;
     Cand bc{layouts[0], 256, 1};
@@ -823,13 +901,22 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
         sc.dyn = h->d_dyn; sc.step_base = h->d_step;
         // ---- exchange, concatenated over replicas
         std::vector<uint32_t> xadj(1, 0), adj;
-        std::vector<double> val9;
+        std::vector<double> val9_all;                     // several replicas: concatenated
+        const double* val9 = nullptr;                     // one: the caller's values as they are
         std::vector<int32_t> doff;
         if (h->exch == ASD_EXCH_CSR) {
+            uint64_t nnz = 0;
             for (uint32_t r = 0; r < nsys; r++) {
                 const asd_system& s = sys[r];
                 REQUIRE(s.xadj && (s.nnz == 0 || (s.adjncy && s.csr_val)), "CSR arrays missing");
                 REQUIRE(s.xadj[0] == 0 && s.xadj[s.nspins] == s.nnz, "xadj must start at 0 and end at nnz");
+                nnz += s.nnz;
+            }
+            xadj.reserve((size_t)n + 1);
+            adj.reserve(nnz);
+            if (nsys > 1) val9_all.reserve(9 * nnz);
+            for (uint32_t r = 0; r < nsys; r++) {
+                const asd_system& s = sys[r];
                 const uint32_t off = h->h_rep_off[r], base = (uint32_t)adj.size();
                 for (uint32_t i = 0; i < s.nspins; i++) {
                     REQUIRE(s.xadj[i + 1] >= s.xadj[i], "xadj must be non-decreasing");
@@ -838,12 +925,13 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
                 for (uint32_t k = 0; k < s.nnz; k++) {
                     REQUIRE(s.adjncy[k] < s.nspins, "adjncy index out of range");
                     adj.push_back(off + s.adjncy[k]);
-                    for (int q = 0; q < 9; q++) {
-                        REQUIRE(std::isfinite(s.csr_val[9 * (size_t)k + q]), "non-finite exchange value");
-                        val9.push_back(s.csr_val[9 * (size_t)k + q]);
-                    }
                 }
+                bool finite = true;
+                for (size_t k = 0; k < 9 * (size_t)s.nnz; k++) finite &= std::isfinite(s.csr_val[k]);
+                REQUIRE(finite, "non-finite exchange value");
+                if (nsys > 1) val9_all.insert(val9_all.end(), s.csr_val, s.csr_val + 9 * (size_t)s.nnz);
             }
+            val9 = nsys > 1 ? val9_all.data() : s0.csr_val;
             h->nnz_per_row = (double)adj.size() / n;
         } else if (h->exch == ASD_EXCH_DIA) {
             REQUIRE(nsys == 1, "DIA exchange supports one replica per handle");
@@ -1017,7 +1105,7 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
                         }
                         cx[i + 1] = (uint32_t)ca.size();
                     }
-                    build_sell(h, cx, ca, cv);
+                    build_sell(h, cx, ca, cv.data());
                     h->dexch = ASD_EXCH_CSR;
                 }
             }
@@ -1083,9 +1171,9 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
         CK(cudaHostAlloc(reinterpret_cast<void**>(&h->h_err), sizeof(uint32_t), cudaHostAllocDefault));
         if (!plain) {
             if (p.flags & ASD_FLAG_AUTOTUNE) autotune(h);
-            else configure_stage(h, 256, 1);
+            else configure_stage(h, 256, (int)STAGE_PATTERN);
             if (h->tune.empty()) {
-                static const char* names[3] = {"direct", "words", "words+spins"};
+                static const char* names[4] = {"direct", "words", "words+spins", "pattern"};
                 char b[64];
                 std::snprintf(b, sizeof b, "block=%d staging=%s (default)", h->block, names[h->sell.stage]);
                 h->tune = b;

@@ -110,21 +110,24 @@ __constant__ double FRK5C[6] = {37.0 / 378.0, 0.0, 250.0 / 621.0, 125.0 / 594.0,
 __constant__ double FRK4C[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
 
 // Register caps of the FP32 kernels: 6 blocks of 256 per SM (40 registers) for the SELL and
-// the field-only kernels, 5 (48) for the DIA kernels; the FP64 kernels keep the default cap.
+// the field-only kernels, 5 (48) for the DIA and the pattern kernels; the FP64 kernels keep the
+// default cap.  The pattern kernels have no staging state and gather six neighbours at once: at 40
+// registers their last stages spill and 96.2 µs per step became 91.6 at 48 (sc 128³, 300 K);
+// at 64 (4 blocks) the large lattices lose (24 replicas 120 → 152 µs per step).
 // At 40 the diagonal-tensor SELL kernels spill 76 bytes a thread (the others none), and still
 // run faster than at 48: the extra warps hide more of the gather's latency than the spills add
 // (96 replicas 564 → 534 µs per step, the north star unchanged, A/B on one box).
 template <typename R, int EX, bool FULL, int K>
 struct MinBlocks {
     static constexpr int value =
-        sizeof(R) != 4 ? 1 : (EX == ASD_EXCH_CSR || EX == ASD_EXCH_NONE) ? 6 : 5;
+        sizeof(R) != 4 ? 1 : (EX == ASD_EXCH_DIA || EX == EXCH_PATTERN) ? 5 : 6;
 };
 
 // K: the stage kind at compile time (1 Heun predictor, 2 Heun corrector, 3 RK stage before the
 // last, 4 last RK stage); a.kind still carries the RK stage index.
 template <typename R, int EX, bool FULL, bool COMP, int K>
 __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
-    stage_kernel(const StepConst c, const SellDev sell, const DiaDev dia, const StageArgs<R> a) {
+    stage_kernel(const StepConst c, const SellDev sell, const PatDev pat, const DiaDev dia, const StageArgs<R> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t stage_bar;
     R* tab = reinterpret_cast<R*>(smem_raw);
@@ -207,6 +210,19 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
     if constexpr (EX == ASD_EXCH_DIA) {
         if (dia.dtype) load_table<R>(table_of<R>(dia), table_stride<FULL>() *dia.ntypes, tab);
     }
+    // Row patterns (PatDev): no words to stage and no wait.  The stage reads 2 bytes of matrix per
+    // row instead of 28 (sc, 6 neighbours) or 108 (BCT-2, 26), and the pattern's entries come
+    // from L1, so all of the row's gathers are issued at once.  Measured against the fastest of the
+    // staged SELL shapes (step time in the graph, one B200): sc 128³ at 300 K 119.2 → 91.6 µs,
+    // 24 sc replicas (2.7 M spins) 155.0 → 121.6, sc 128×128×64 with dipole 175.9 → 163.0, BCT-2
+    // 64³ 55.4 → 49.2, sc 16³ 8.9 → 7.7.
+    uint32_t pid = 0;
+    if constexpr (EX == EXCH_PATTERN) {
+        const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
+        if (row < c.n) pid = __ldg(pat.row + row);
+        if constexpr (FULL) load_table<R>(table_of<R>(sell), table_stride<FULL>() * sell.ntypes, tab);
+        else tab = const_cast<R*>(table_of<R>(sell));
+    }
     pdl_enter();
     if constexpr (EX == ASD_EXCH_CSR) {
         // the neighbour-spin spans: one copy per (span, component), on the staging barrier
@@ -284,8 +300,13 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
         stage_timeout = true;
     }
     R h[3] = {R(0), R(0), R(0)};
+    // stage spin at this site; the pattern kernels load it with the gather's first loads
+    R sv[3];
+    if constexpr (EX == EXCH_PATTERN)
+        for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
     if constexpr (EX == ASD_EXCH_CSR) gather_sell<R, FULL>(sell, i, a.src, tab, h, staged, wbase, sspin, staged16);
     if constexpr (EX == ASD_EXCH_DIA) gather_dia<R, FULL>(dia, c.n, i, a.src, tab, h);
+    if constexpr (EX == EXCH_PATTERN) gather_pattern<R, FULL>(pat, pid, i, a.src, tab, h);
     if (c.q4_ptr) {
         R h4[3];
         four_spin<R>(c, i, [&](uint32_t j, R v[3]) { v[0] = a.src.p[0][j]; v[1] = a.src.p[1][j]; v[2] = a.src.p[2][j]; }, h4);
@@ -309,8 +330,8 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
     h[1] += lrn[1] + dynr[DYN_APPLIED + 1];
     h[2] += lrn[2] + dynr[DYN_APPLIED + 2];
 
-    // stage spin at this site
-    R sv[3] = {a.src.p[0][i], a.src.p[1][i], a.src.p[2][i]};
+    if constexpr (EX != EXCH_PATTERN)
+        for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
     const int kind = a.kind;
     if constexpr (K >= 3) {
         if (kind >= 11 && (c.flags & ASD_FLAG_RK_STAGE_SPIN_MIXED)) sv[1] = a.base.p[1][i];
@@ -437,7 +458,8 @@ double stage_bytes(const asd_handle* h, const StageArgs<R>& a, bool comp) {
     const double vb = sizeof(R), n = h->n;
     const double c = h->full ? 9.0 : 3.0;
     double m = 0.0;
-    if (h->dexch == ASD_EXCH_CSR) m = 4.0 + h->nnz_per_row * (h->sell.typed ? 4.0 : 4.0 + vb * c);
+    if (h->dexch == ASD_EXCH_CSR && h->sell.stage == STAGE_PATTERN) m = 2.0;
+    else if (h->dexch == ASD_EXCH_CSR) m = 4.0 + h->nnz_per_row * (h->sell.typed ? 4.0 : 4.0 + vb * c);
     else if (h->dexch == ASD_EXCH_DIA) m = h->nnz_per_row * (h->dia.dtype ? 1.0 : vb * c);
     double st = 3 * vb;                                  // src spin (gathered once)
     const int kind = a.kind;
@@ -475,6 +497,7 @@ cudaError_t launch_stage_k(asd_handle* hd, const StageArgs<R>& a) {
             smem = ((smem + 15) & ~(size_t)15) + 4 * (size_t)hd->sell.stage_words;
         if (hd->sell.stage == 2) smem += 3 * sizeof(R) * (size_t)hd->sell.spin_slots;
     }
+    if (EX == EXCH_PATTERN && FULL) smem = sizeof(R) * table_stride<FULL>() * hd->sell.ntypes;
     if (EX == ASD_EXCH_DIA && hd->dia.dtype) smem = sizeof(R) * table_stride<FULL>() *hd->dia.ntypes;
     {
         const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(stage_kernel<R, EX, FULL, COMP, K>), smem);
@@ -483,14 +506,14 @@ cudaError_t launch_stage_k(asd_handle* hd, const StageArgs<R>& a) {
     timer_begin(hd);
     {
         const cudaError_t e = launch_step_kernel(stage_kernel<R, EX, FULL, COMP, K>, dim3(grid), dim3(B), smem,
-                                                 hd->stream, 1, step_pdl(hd), hd->sc, hd->sell, hd->dia, a);
+                                                 hd->stream, 1, step_pdl(hd), hd->sc, hd->sell, hd->pat, hd->dia, a);
         if (e != cudaSuccess) return e;
     }
     hd->launches += 1;
     if (hd->timing) {
-        const bool typed = (EX == ASD_EXCH_CSR && hd->sell.typed) || (EX == ASD_EXCH_DIA && hd->dia.dtype);
+        const bool typed = (EX == ASD_EXCH_CSR && hd->sell.typed) || EX == EXCH_PATTERN || (EX == ASD_EXCH_DIA && hd->dia.dtype);
         const std::string name = std::string("stage_kernel<") + (sizeof(R) == 4 ? "float" : "double") + "," +
-                                 (EX == ASD_EXCH_CSR ? "SELL32" : EX == ASD_EXCH_DIA ? "DIA" : "NONE") +
+                                 (EX == ASD_EXCH_CSR ? "SELL32" : EX == EXCH_PATTERN ? "pattern" : EX == ASD_EXCH_DIA ? "DIA" : "NONE") +
                                  (typed ? "-typed" : "") + (FULL ? ",full" : ",diag") + (COMP ? ",comp" : "") +
                                  (K == 1 ? ",predictor>" : K == 2 ? ",corrector>" : K == 3 ? ",rk-stage>" : ",rk-last>");
         timer_end(hd, name, stage_bytes<R>(hd, a, COMP));
@@ -508,7 +531,9 @@ cudaError_t launch_stage_t(asd_handle* hd, const StageArgs<R>& a) {
 
 template <typename R, bool COMP>
 cudaError_t launch_stage(asd_handle* hd, const StageArgs<R>& a) {
-    if (hd->dexch == ASD_EXCH_CSR) {
+    if (hd->dexch == ASD_EXCH_CSR && hd->sell.stage == STAGE_PATTERN) {
+        return hd->full ? launch_stage_t<R, EXCH_PATTERN, true, COMP>(hd, a) : launch_stage_t<R, EXCH_PATTERN, false, COMP>(hd, a);
+    } else if (hd->dexch == ASD_EXCH_CSR) {
         return hd->full ? launch_stage_t<R, ASD_EXCH_CSR, true, COMP>(hd, a) : launch_stage_t<R, ASD_EXCH_CSR, false, COMP>(hd, a);
     } else if (hd->dexch == ASD_EXCH_DIA) {
         return hd->full ? launch_stage_t<R, ASD_EXCH_DIA, true, COMP>(hd, a) : launch_stage_t<R, ASD_EXCH_DIA, false, COMP>(hd, a);

@@ -228,6 +228,22 @@ __device__ __forceinline__ void gather_sell(const SellDev& m, uint32_t i, const 
     }
 }
 
+// h += sum over the row's pattern of J_id S_{i + delta}; `tab` is the tensor table (global memory
+// for the diagonal form, whose few rows stay in L1; shared memory for full tensors).
+template <typename R, bool FULL>
+__device__ __forceinline__ void gather_pattern(const PatDev& m, uint32_t pid, uint32_t i, const CVec3<R>& s,
+                                               const R* tab, R h[3]) {
+    const int2* __restrict__ e = m.ent + (size_t)pid * m.W;
+    const uint32_t W = m.W;
+#pragma unroll 6
+    for (uint32_t k = 0; k < W; k++) {
+        const int2 v = __ldg(e + k);
+        const uint32_t j = i + (uint32_t)v.x;
+        const R x = __ldg(s.p[0] + j), y = __ldg(s.p[1] + j), z = __ldg(s.p[2] + j);
+        accumulate_typed<R, FULL>(tab, (uint32_t)v.y, x, y, z, h);
+    }
+}
+
 // h += sum over diagonals d with 0 <= i+off[d] < n of J_{d,i} S_{i+off[d]}, row-aligned DIA.
 template <typename R, bool FULL>
 __device__ __forceinline__ void gather_dia(const DiaDev& m, uint32_t n, uint32_t i, const CVec3<R>& s, const R* tab,

@@ -48,6 +48,18 @@ struct SellDev {
     uint4* spans = nullptr;          // (start, len, off, 0) in elements
     uint32_t spin_slots = 0, spin_block = 0;
 };
+// Row patterns of a typed matrix: the distinct sequences of (column - row, tensor id) over its
+// rows (a regular lattice has one per sublattice and boundary situation).  A row then costs its
+// 2-byte pattern number; the sequences, padded to W entries with (0, zero tensor), are read
+// through L1 by every row that follows them.  Entries keep the SELL order.
+struct PatDev {
+    uint32_t W = 0;                  // entries per pattern (0: no patterns)
+    uint32_t npat = 0;
+    uint16_t* row = nullptr;         // pattern of each row
+    int2* ent = nullptr;             // [npat][W]: (column - row, tensor id)
+};
+constexpr uint32_t STAGE_PATTERN = 3;   // SellDev::stage: the stage kernels gather by row patterns
+constexpr int EXCH_PATTERN = 4;         // the stage kernel's layout parameter in that mode
 constexpr uint32_t MAG_CHUNK = 2048;  // spins per block of the magnetisation reduction
 constexpr uint32_t SPIN_PAD = 8;     // zeroed elements after every gather-source spin array
 
@@ -175,6 +187,7 @@ struct asd_handle {
     double* nzd[3] = {nullptr};
     double *detd[3] = {nullptr}, *stagd[3] = {nullptr};
     asd::SellDev sell;
+    asd::PatDev pat;
     asd::DiaDev dia;
     // FP64 plain (AoS [3i+c], reference-structured)
     double *p_s = nullptr, *p_es = nullptr, *p_fn = nullptr, *p_ch = nullptr, *p_hdemag = nullptr, *p_rand = nullptr,
