@@ -405,16 +405,13 @@ void setup_lr(asd_handle* h, const asd_system& s, bool plain) {
     L.P = (size_t)L.mesh[0] * L.mesh[1] * L.mesh[2];
     L.Pk = (size_t)L.mesh[0] * L.mesh[1] * (L.mesh[2] / 2 + 1);
     REQUIRE(s.mesh_xyz && s.nr, "long-range field needs mesh_xyz and nr");
-    std::vector<uint32_t> idx(h->n);
     std::vector<float> w(h->n);
     for (uint32_t i = 0; i < h->n; i++) {
         const uint32_t x = s.mesh_xyz[3 * i], y = s.mesh_xyz[3 * i + 1], z = s.mesh_xyz[3 * i + 2];
         REQUIRE(x < L.mesh[0] && y < L.mesh[1] && z < L.mesh[2], "mesh_xyz outside the mesh");
-        idx[i] = (uint32_t)(((size_t)x * L.mesh[1] + y) * L.mesh[2] + z);
         const uint32_t at = s.atom ? s.atom[i] : i % s.nmat;
         w[i] = s.lr == ASD_LR_DIPOLE ? (float)s.mat[at].mu : 1.0f;
     }
-    L.mesh_idx = dupload(idx.data(), idx.size());
     L.w = dupload(w.data(), w.size());
     // symmetry of N_r (up to rounding of (3 e_a) e_b) decides 6 or 9 stored components;
     // a symmetric matrix is stored as the mean of each (a,b),(b,a) pair
@@ -458,7 +455,84 @@ void setup_lr(asd_handle* h, const asd_system& s, bool plain) {
                     }
         }
     }
-    double* d_nr = dupload(plain ? s.nr : nrs.data(), 9 * L.P);
+    // The plane kernels where their axis lengths, the box and the shared memory fit; a complex N_k
+    // must fit as well unless N_r is even over the box (then N_k is real).
+    const uint32_t box[3] = {hi[0] - lo[0] + 1, hi[1] - lo[1] + 1, hi[2] - lo[2] + 1};
+    auto even = [&]() {
+        if (!sym) return false;
+        for (uint32_t x = 0; x < box[0]; x++)
+            for (uint32_t y = 0; y < 2 * box[1] - 1; y++)
+                for (uint32_t z = 0; z < 2 * box[2] - 1; z++) {
+                    const uint32_t dy = y < box[1] ? y : s.mesh[1] - (y - box[1] + 1);
+                    const uint32_t dz = z < box[2] ? z : s.mesh[2] - (z - box[2] + 1);
+                    const uint32_t c[3] = {x, dy, dz};
+                    size_t at = 0, mir = 0;
+                    for (int a = 0; a < 3; a++) {
+                        at = at * s.mesh[a] + c[a];
+                        mir = mir * s.mesh[a] + (c[a] ? s.mesh[a] - c[a] : 0);
+                    }
+                    for (int q = 0; q < 9; q++)
+                        if (std::fabs(nrs[q * L.P + at] - nrs[q * L.P + mir]) > 1e-13 * amax) return false;
+                }
+        return true;
+    };
+    auto fits = [&](const LongRange& l) {
+        return plane_path_fits(l, false) && (plane_path_fits(l, true) || even());
+    };
+    uint32_t org[3] = {0, 0, 0};                       // mesh position of the caller's origin, negated
+    if (!plain && h->n > 0 && !(h->p.flags & ASD_FLAG_CUFFT_PLANES)) {
+        for (int a = 0; a < 3; a++) { L.box0[a] = lo[a]; L.box1[a] = hi[a]; }
+        L.planes = fits(L) ? 1 : 0;
+        // Another mesh: where no two spins of the box alias on the caller's mesh, its N_r holds
+        // every interaction at one displacement each, and the convolution is the same on any mesh
+        // of at least twice the box.  A mesh whose axes are not lengths of the plane kernels
+        // (2 L for a ragged L) moves to the shortest that are.  cuFFT's 3D transforms of the
+        // caller's mesh cannot skip the zero-padding, run strictly in order and fall to slow
+        // radices.  Measured (µs per step of the sc lattice with dipole, caller's mesh by cuFFT → moved):
+        // 90×75×41 (180×150×82 → 192×192×96) 207.9 → 69.7, 100×100×60 274.8 → 132.1, 30³ 33.0 →
+        // 19.9, 20×25×9 25.5 → 17.8, 120×100×3 37.9 → 33.6.  A power-of-two mesh of 2 or 4 z points
+        // (films of one or two layers) stays: the plane kernels' shortest z axis is 8, and cuFFT's
+        // power-of-two planes win (128×128×1 31.3 against 34.3).
+        const bool p2 = !((L.mesh[0] & (L.mesh[0] - 1)) | (L.mesh[1] & (L.mesh[1] - 1)) | (L.mesh[2] & (L.mesh[2] - 1)));
+        bool alone = true;
+        for (int a = 0; a < 3; a++) alone &= 2 * box[a] <= L.mesh[a] + 1;
+        if (!L.planes && alone && !(p2 && L.mesh[2] <= 4)) {
+            LongRange t = L;
+            plane_mesh_for(box, t.mesh);
+            for (int a = 0; a < 3; a++) { t.box0[a] = 0; t.box1[a] = box[a] - 1; }
+            if (t.mesh[0] && t.mesh[1] && t.mesh[2] && fits(t)) {
+                L = t;
+                L.planes = 1;
+                L.P = (size_t)L.mesh[0] * L.mesh[1] * L.mesh[2];
+                L.Pk = (size_t)L.mesh[0] * L.mesh[1] * (L.mesh[2] / 2 + 1);
+                for (int a = 0; a < 3; a++) org[a] = lo[a];
+            }
+        }
+    }
+    const bool moved = L.mesh[0] != s.mesh[0] || L.mesh[1] != s.mesh[1] || L.mesh[2] != s.mesh[2];
+    {
+        std::vector<uint32_t> idx(h->n);
+        for (uint32_t i = 0; i < h->n; i++)
+            idx[i] = (uint32_t)(((size_t)(s.mesh_xyz[3 * i] - org[0]) * L.mesh[1] + (s.mesh_xyz[3 * i + 1] - org[1])) * L.mesh[2] +
+                                (s.mesh_xyz[3 * i + 2] - org[2]));
+        L.mesh_idx = dupload(idx.data(), idx.size());
+    }
+    double* d_nr = dupload(plain ? s.nr : nrs.data(), nrs.size());
+    if (moved) {
+        // (not dalloc: its zeroing runs on the default stream, which h->stream does not wait for;
+        // embed_nr zeroes on h->stream)
+        double* d = nullptr;
+        cudaError_t em = cudaMalloc(&d, sizeof(double) * 9 * L.P);
+        if (em == cudaSuccess) em = embed_nr(h, box, s.mesh, L.mesh, d_nr, d);
+        const cudaError_t es = cudaStreamSynchronize(h->stream);
+        cudaFree(d_nr);
+        d_nr = d;
+        if (em != cudaSuccess || es != cudaSuccess) {
+            cudaFree(d_nr);
+            CK(em);
+            CK(es);
+        }
+    }
     int dims[3] = {(int)L.mesh[0], (int)L.mesh[1], (int)L.mesh[2]};
     cudaError_t e;
     if (plain) {
@@ -475,10 +549,6 @@ void setup_lr(asd_handle* h, const asd_system& s, bool plain) {
         // pruned transform when the last axis is a power of two: z transforms only for the rows
         // of the spins' box, 2D transforms of the (x, y) planes by cuFFT
         L.pruned = (mz >= 4 && mz <= 2048 && (mz & (mz - 1)) == 0 && h->n > 0) ? 1 : 0;   // z-pass smem <= 45 KB
-        if (L.pruned) for (int a = 0; a < 3; a++) { L.box0[a] = lo[a]; L.box1[a] = hi[a]; }
-        // the library's plane kernels replace cuFFT's (x, y) passes where every axis fits them
-        L.planes = (L.pruned && !(h->p.flags & ASD_FLAG_CUFFT_PLANES) && plane_path_fits(L, false) &&
-                    plane_path_fits(L, true)) ? 1 : 0;
         if (L.planes) {
             // buffers are allocated with the tiled N_k (build_nk_f32)
         } else if (L.pruned) {

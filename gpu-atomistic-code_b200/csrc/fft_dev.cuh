@@ -1,7 +1,8 @@
 // Device building blocks of the long-range-field transforms (FP32, power-of-two sizes).
 //
-//  * dft<R, INV>: R-point DFT (R <= 16) of a register array, natural order in and out,
-//    radix-4/radix-2 with compile-time twiddles (multiplications by +-1, +-i are free).
+//  * dft<R, INV>: R-point DFT (R = 2, 3, 4, 6, 8, 12, 16) of a register array, natural
+//    order in and out, from radix 4, 2 and 3 with compile-time twiddles (multiplications by +-1,
+//    +-i are free).
 //  * The "four-step" split N = R1 R2 used by the plane kernels:
 //        X[m + R1 q] = sum_t w_R2^{t q} w_N^{t m} sum_k w_R1^{k m} x[t + R2 k]
 //    pass 1: one thread per t runs the R1-point DFT over k and multiplies by w_N^{t m};
@@ -11,6 +12,7 @@
 //    z_n = x_2n + i x_2n+1 plus the split) with its shared-memory two-pass FFT.
 #pragma once
 #include <cstdint>
+#include <type_traits>
 
 namespace asd {
 namespace fftd {
@@ -32,6 +34,11 @@ __device__ __forceinline__ float2 tw16(float2 a, int e) {
     constexpr float C1 = 0.92387953251128676f;   // cos(pi/8)
     constexpr float S1 = 0.38268343236508977f;   // sin(pi/8)
     constexpr float H = 0.70710678118654752f;    // sqrt(1/2)
+    // C1 and H round down: with them alone a convolution (three axes, there and back) comes out 9e-8
+    // too small on average, the same at every step.  Half of the C1 twiddles and the real part of
+    // w_16^6 take the next float above, which leaves less than 1e-8 (mean gain of the passes on a box of
+    // half the axis, per axis there and back: 64 points -2.0e-8 → -0.1e-8, 256 -2.9e-8 → 0.2e-8).
+    constexpr float C1U = 0.92387956380844116f, HU = 0.70710682868957520f;
     const float sg = INV ? 1.0f : -1.0f;         // sign of the imaginary part of w_16^1
     switch (e & 15) {
     case 0: return a;
@@ -39,17 +46,57 @@ __device__ __forceinline__ float2 tw16(float2 a, int e) {
     case 8: return make_float2(-a.x, -a.y);
     case 12: return INV ? make_float2(a.y, -a.x) : make_float2(-a.y, a.x);
     case 2: return cmul(a, make_float2(H, sg * H));
-    case 6: return cmul(a, make_float2(-H, sg * H));
+    case 6: return cmul(a, make_float2(-HU, sg * H));
     case 10: return cmul(a, make_float2(-H, -sg * H));
     case 14: return cmul(a, make_float2(H, -sg * H));
-    case 1: return cmul(a, make_float2(C1, sg * S1));
+    case 1: return cmul(a, make_float2(C1U, sg * S1));
     case 3: return cmul(a, make_float2(S1, sg * C1));
     case 5: return cmul(a, make_float2(-S1, sg * C1));
     case 7: return cmul(a, make_float2(-C1, sg * S1));
-    case 9: return cmul(a, make_float2(-C1, -sg * S1));
+    case 9: return cmul(a, make_float2(-C1U, -sg * S1));
     case 11: return cmul(a, make_float2(-S1, -sg * C1));
     case 13: return cmul(a, make_float2(S1, -sg * C1));
     default: return cmul(a, make_float2(C1, -sg * S1));   // 15
+    }
+}
+
+// cos(2 pi e / R) and sin(2 pi e / R), 0 <= e < R, evaluated by the compiler in double precision
+// (Taylor series on [0, pi / 4], the octants by symmetry).
+__host__ __device__ constexpr double series_cs(double x, bool sine) {
+    double t = sine ? x : 1.0, s = 0.0;
+    for (int k = sine ? 1 : 0; k < 30; k += 2) { s += t; t *= -x * x / ((k + 1) * (k + 2)); }
+    return s;
+}
+__host__ __device__ constexpr double cos_turn(int e, int R) {
+    constexpr double PI = 3.14159265358979323846;
+    if (2 * e > R) e = R - e;                              // cos is even
+    if (4 * e > R) return -cos_turn(R - 2 * e, 2 * R);     // cos(pi - x)
+    return 8 * e > R ? series_cs(2 * PI * (R - 4 * e) / (4.0 * R), true) : series_cs(2 * PI * e / R, false);
+}
+__host__ __device__ constexpr double sin_turn(int e, int R) {
+    return cos_turn((4 * e + 3 * R) % (4 * R), 4 * R);     // cos(x - pi / 2)
+}
+
+// a * w_R^E (forward, w = exp(-2 pi i / R)) or a * conj(w_R^E) (inverse).
+template <int R, bool INV, int E>
+__device__ __forceinline__ float2 twc(float2 a) {
+    constexpr int e = E % R;
+    if constexpr (e == 0) return a;
+    else if constexpr (4 * e == R) return INV ? make_float2(-a.y, a.x) : make_float2(a.y, -a.x);
+    else if constexpr (2 * e == R) return make_float2(-a.x, -a.y);
+    else if constexpr (4 * e == 3 * R) return INV ? make_float2(a.y, -a.x) : make_float2(-a.y, a.x);
+    else {
+        constexpr float c = (float)cos_turn(e, R), s = (float)sin_turn(e, R);
+        return cmul(a, make_float2(c, INV ? s : -s));
+    }
+}
+
+// f(integral_constant<int, K>) for K = 0 .. N - 1, unrolled.
+template <int N, int K = 0, typename F>
+__device__ __forceinline__ void static_for(F&& f) {
+    if constexpr (K < N) {
+        f(std::integral_constant<int, K>{});
+        static_for<N, K + 1>(f);
     }
 }
 
@@ -88,29 +135,76 @@ struct Dft<4, INV> {
     }
 };
 
+template <bool INV>
+struct Dft<3, INV> {
+    static __device__ __forceinline__ void run(float2* v) {
+        // sin(2 pi / 3) rounded up, against the other constants' rounding down (tw16): mean gain of
+        // 48 points -1.5e-8 → 0.0e-8, 192 points -1.3e-8 → 0.4e-8
+        constexpr float S3 = 0.86602544784545898f;
+        const float2 t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
+        const float2 m = make_float2(v[0].x - 0.5f * t.x, v[0].y - 0.5f * t.y);
+        const float2 s = mul_mi<INV>(make_float2(S3 * d.x, S3 * d.y));
+        v[0] = cadd(v[0], t);
+        v[1] = cadd(m, s);
+        v[2] = csub(m, s);
+    }
+};
+
+// R = 6, 12: four-step N1 x 3 with N1 = 2 or 4.
+template <int R, bool INV>
+__device__ __forceinline__ void dft_mixed(float2* v) {
+    constexpr int N1 = R / 3, Q = 3;
+    float2 a[Q][N1];
+    static_for<Q>([&](auto tc) {
+        constexpr int t = decltype(tc)::value;
+#pragma unroll
+        for (int k = 0; k < N1; k++) a[t][k] = v[t + Q * k];
+        Dft<N1, INV>::run(a[t]);
+        static_for<N1>([&](auto mc) {
+            constexpr int m = decltype(mc)::value;
+            a[t][m] = twc<R, INV, t * m>(a[t][m]);
+        });
+    });
+#pragma unroll
+    for (int m = 0; m < N1; m++) {
+        float2 b[Q];
+#pragma unroll
+        for (int t = 0; t < Q; t++) b[t] = a[t][m];
+        Dft<Q, INV>::run(b);
+#pragma unroll
+        for (int q = 0; q < Q; q++) v[m + N1 * q] = b[q];
+    }
+}
+template <int R>
+__host__ __device__ constexpr bool mixed_radix() { return R == 6 || R == 12; }
+
 // R = 4 Q (Q = 2 or 4): four-step with N1 = 4, N2 = Q in registers.
 template <int R, bool INV>
 struct Dft {
-    static_assert(R == 8 || R == 16, "register DFT sizes are 1, 2, 4, 8, 16");
+    static_assert(R == 8 || R == 16 || mixed_radix<R>(), "register DFT sizes are 1, 2, 3, 4, 6, 8, 12, 16");
     static __device__ __forceinline__ void run(float2* v) {
-        constexpr int Q = R / 4;
-        float2 a[Q][4];
+        if constexpr (mixed_radix<R>()) {
+            dft_mixed<R, INV>(v);
+        } else {
+            constexpr int Q = R / 4;
+            float2 a[Q][4];
 #pragma unroll
-        for (int t = 0; t < Q; t++) {
+            for (int t = 0; t < Q; t++) {
 #pragma unroll
-            for (int k = 0; k < 4; k++) a[t][k] = v[t + Q * k];
-            Dft<4, INV>::run(a[t]);
+                for (int k = 0; k < 4; k++) a[t][k] = v[t + Q * k];
+                Dft<4, INV>::run(a[t]);
 #pragma unroll
-            for (int m = 1; m < 4; m++) a[t][m] = tw16<INV>(a[t][m], (t * m) * (16 / R));
-        }
+                for (int m = 1; m < 4; m++) a[t][m] = tw16<INV>(a[t][m], (t * m) * (16 / R));
+            }
 #pragma unroll
-        for (int m = 0; m < 4; m++) {
-            float2 b[Q];
+            for (int m = 0; m < 4; m++) {
+                float2 b[Q];
 #pragma unroll
-            for (int t = 0; t < Q; t++) b[t] = a[t][m];
-            Dft<Q, INV>::run(b);
+                for (int t = 0; t < Q; t++) b[t] = a[t][m];
+                Dft<Q, INV>::run(b);
 #pragma unroll
-            for (int q = 0; q < Q; q++) v[m + 4 * q] = b[q];
+                for (int q = 0; q < Q; q++) v[m + 4 * q] = b[q];
+            }
         }
     }
 };
@@ -187,15 +281,17 @@ struct DftP {
 };
 
 // The R-point DFT with the upper half of the inputs zero (HIN) and/or only the lower half of the
-// outputs formed (HOUT).
+// outputs needed (HOUT; of a size with a factor 3 the compiler drops the others).
 template <int R, bool INV, bool HIN, bool HOUT>
 __device__ __forceinline__ void dftp(float2 (&v)[R]) {
-    if constexpr (!HIN && !HOUT) Dft<R, INV>::run(v);
+    static_assert(!HIN || R % 3 != 0, "pass 1 runs powers of two");
+    if constexpr ((!HIN && !HOUT) || R % 3 == 0) Dft<R, INV>::run(v);
     else DftP<R, INV, HIN ? R / 2 : R, HOUT ? R / 2 : R>::run(v);
 }
 
-// (R1, R2) of the four-step split of a power-of-two N <= 256 (R1 >= R2).
-__host__ __device__ constexpr int split_r1(int N) { return N <= 2 ? N : N <= 8 ? (N == 8 ? 4 : 2) : N <= 32 ? (N == 32 ? 8 : 4) : N <= 128 ? (N == 128 ? 16 : 8) : 16; }
+// (R1, R2) of the four-step split: a power of two N <= 256, or 24, 48, 96, 192 (R1 >= R2; R1 a
+// power of two, so that the half-zero inputs and half-formed outputs are whole rows k of pass 1).
+__host__ __device__ constexpr int split_r1(int N) { return N % 3 == 0 ? (N <= 48 ? 8 : 16) : N <= 2 ? N : N <= 8 ? (N == 8 ? 4 : 2) : N <= 32 ? (N == 32 ? 8 : 4) : N <= 128 ? (N == 128 ? 16 : 8) : 16; }
 __host__ __device__ constexpr int split_r2(int N) { return N / split_r1(N); }
 __host__ __device__ constexpr uint32_t ilog2c(uint32_t v) { return v <= 1 ? 0 : 1 + ilog2c(v / 2); }
 
@@ -234,13 +330,13 @@ __host__ __device__ constexpr bool rows_warp_local() { return N1 == N2 && 32 % N
 // N = N1 * N2 point DFT of TY rows of shared memory (row pitch ld, natural order in and out, in
 // place), TY * max(N1, N2) <= blockDim.x; N1, N2 <= 16.  The intermediate between the passes is
 // stored with pitch N2 + 1 per m, so ld >= N1 (N2 + 1); with ld = N2 (mod 16) the accesses of
-// both passes are free of bank conflicts.  Ends with a barrier: the warp's when
+// both passes are free of bank conflicts (powers of two).  Ends with a barrier: the warp's when
 // rows_warp_local<N1, N2>() (the caller then writes and reads each row from the warp owning
 // it), else the block's.
 template <int N1, int N2, bool INV, bool HIN = false, bool HOUT = false>
 __device__ __forceinline__ void fft2pass(float2* s, uint32_t ld, const float2* tw, uint32_t TY) {
     // HIN: the row's inputs N/2..N are zero (pass 1 reads k < N1/2 only); HOUT: only the outputs
-    // 0..N/2 are formed (pass 2 writes q < N2/2 only)
+    // 0..N/2 are needed (pass 2 writes q < N2/2, rounded up)
     constexpr bool WL = rows_warp_local<N1, N2>();
     {
         const uint32_t it = threadIdx.x, r = it / N2, t = it % N2;
@@ -272,7 +368,7 @@ __device__ __forceinline__ void fft2pass(float2* s, uint32_t ld, const float2* t
         group_sync<WL>();
         if (act) {
 #pragma unroll
-            for (int q = 0; q < (HOUT ? N2 / 2 : N2); q++) s[r * ld + m + N1 * q] = u[q];
+            for (int q = 0; q < (HOUT ? (N2 + 1) / 2 : N2); q++) s[r * ld + m + N1 * q] = u[q];
         }
         group_sync<WL>();
     }

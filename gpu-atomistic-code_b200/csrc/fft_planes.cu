@@ -15,11 +15,12 @@
 //
 // Shifting the box to the origin along x and y does not change the cyclic convolution (it
 // depends on mesh differences only), and lets every pass skip the zero half of its input and
-// the discarded half of its output.  The transforms are unnormalised like cuFFT's: the stage
-// kernels multiply the gathered field by 1/P.
+// the discarded half of its output.  The transforms are unnormalised like cuFFT's; N_k carries
+// the factor 1/P.
 #include "fft_dev.cuh"
 #include "gather.cuh"
 #include <algorithm>
+#include <cmath>
 #include <cooperative_groups.h>
 #include <cstring>
 
@@ -36,6 +37,7 @@ struct PlaneArgs {
     uint32_t m0;                     // mesh x (y and z are compile-time in the kernels)
     uint32_t bx0, by0;               // box origin (x, y)
     uint32_t zs, nz;                 // z rows: float2 pairs [zs, zs + nz) hold data, nz <= N/2
+    uint32_t cl;                     // blocks per cluster of the z/y kernels
     uint32_t bx, by;                 // box extents along x (<= m0/2) and y (<= m1/2)
     uint32_t ntile;                  // ky tiles (m1 / PT)
     uint32_t kzb;                    // kz values per y-pass round (rounds balanced)
@@ -51,16 +53,6 @@ struct PlaneArgs {
 };
 
 constexpr uint32_t ERR_FFT_TIMEOUT = 2u;
-
-__device__ __forceinline__ void bulk_store(void* gdst, const void* ssrc, uint32_t bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_addr(ssrc)),
-                 "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_commit_wait_read() {
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-}
 
 // Y element (c, kz, x, ky) in the tiled spectrum layout [c][kz][ky / PT][x][ky % PT].
 __device__ __forceinline__ size_t yk_index(const PlaneArgs& A, uint32_t Kz, uint32_t c, uint32_t kz, uint32_t x,
@@ -85,20 +77,48 @@ struct YkCol {
     __device__ __forceinline__ float2& operator[](uint32_t q) const { return p[q * qs]; }
 };
 
+// Blocks of a cluster that share one box row (CL) in the z/y kernels, for R1 x R2-point y axes,
+// N-point z rows and `rows` box rows (of three components) in the launch.  A block's work goes with
+// N M1 / CL points: one block per row spends the least on the cluster's barriers and remote
+// reads, but runs a wide row's passes one after another in eight warps.  So one block where its row
+// is at most 2048 points, or 8192 when there are rows for more than two blocks per SM; two up to
+// 16,384 points unless the rows are fewer than the SMs; else four.  Measured (µs per step of the sc
+// lattice with dipole, one B200; CL = 1 / 2 / 4, by rows and N M1):
+//   384 rows: 4096 (128×128×16) 56.5 / - / 68.3, 8192 (×32) 86.1 / 89.6 / 94.8, 16384 (×64)
+//   177.5 / 159.3 / 162.9; 300: 2048 (100×30×30) 32.7 / 34.9 / 44.3, 4096 (100×60×30) 50.0 / 47.5 /
+//   56.5; 270: 9216 (90×75×41) 81.3 / 70.0 / 76.8; 192: 4096 (64×64×32) 44.5 / 36.3 / 42.7, 8192
+//   (64³) 71.4 / 52.8 / 59.4; 180: 32768 (60×100×100) 194 / 159 / 148; 120: 4096 (40×100×12) 41.1
+//   / 32.4 / 31.2; 90: 8192 (30×100×30) 52.4 / 41.8 / 33.3; 60: 8192 (20×60×60) 56.4 / 38.1 / 32.8.
+inline uint32_t zy_cl(uint32_t N, uint32_t m1, uint32_t r1, uint32_t rows) {
+    const uint32_t pts = N * m1, most = std::min(r1 / 2, 4u);   // a block's y rows are whole columns of the y pass
+    const uint32_t cl = pts <= (rows > 320 ? 8192u : 2048u) ? 1 : rows > 148 && pts <= 16384 ? 2 : 4;
+    return std::min(cl, most);
+}
+// The values of CL the rule can give: the kernels that are compiled.
+__host__ __device__ constexpr bool zy_cl_used(uint32_t N, uint32_t m1, uint32_t r1, uint32_t cl) {
+    const uint32_t pts = N * m1, most = r1 / 2 < 4 ? r1 / 2 : 4;
+    return cl <= most && (cl == 1 ? pts <= 8192 : cl == 2 ? pts > 2048 && (pts <= 16384 || most == 2) : pts > 2048);
+}
+// k of index n in [0, N]: n mod N.
+template <uint32_t N>
+__device__ __forceinline__ uint32_t mod_n(uint32_t n) {
+    if constexpr ((N & (N - 1)) == 0) return n & (N - 1); else return n == N ? 0 : n;
+}
+
 // Compile-time geometry of the z/y kernels: z rows of N = Z1 Z2 complex points (mesh z = 2N),
 // y transforms of M1 = R1 R2 points.  A (component, box row x) is shared by a cluster of CL
 // blocks: block `rank` transforms the z rows y in [rank HY, rank HY + HY) (the box's y extent
 // is at most M1/2 = CL HY) and the kz in [rank HK, rank HK + HK); the transposed z spectrum of
 // its rows, Zs[KZ][LDZ], is read and written across the cluster in distributed shared memory.
 // HY is a multiple of R2, so the block owning row t + R2 k of a y pass is k / (HY / R2).
-template <int Z1, int Z2, int R1, int R2>
+template <int Z1, int Z2, int R1, int R2, int CLUSTER>
 struct ZYGeom {
     static constexpr uint32_t N = Z1 * Z2, KZ = N + 1;
     static constexpr uint32_t TY = 256 / (Z1 > Z2 ? Z1 : Z2);         // z rows per round
     static constexpr uint32_t LD = fft2pass_pitch(N, Z1, Z2);          // z row pitch
     static constexpr uint32_t M1 = R1 * R2;
-    static constexpr uint32_t CL = M1 >= 32 ? 4 : 1;
-    static constexpr uint32_t HY = M1 >= 32 ? M1 / 8 : M1 / 2;
+    static constexpr uint32_t CL = CLUSTER;
+    static constexpr uint32_t HY = M1 / (2 * CL);
     static constexpr uint32_t KPB = HY / R2;                           // k values per owner block
     static constexpr uint32_t LDZ = HY | 1u;
     // the real kz = 0 and kz = N planes share one complex y transform (slot 0): N slots in all
@@ -106,8 +126,10 @@ struct ZYGeom {
     static_assert(CL == 1 || HY % R2 == 0, "cluster rows must be whole y-pass columns");
     static_assert(N % CL == 0, "y-pass slots split evenly over the cluster");
 };
-__host__ __device__ constexpr uint32_t zy_cl(uint32_t m1) { return m1 >= 32 ? 4 : 1; }
-__host__ __device__ constexpr uint32_t zy_hy(uint32_t m1) { return m1 >= 32 ? m1 / 8 : m1 / 2; }
+// Blocks per SM of the z/y kernels: 4 (64 registers, no spill) where the z rows are at most 64
+// points, 3 for the longer rows, whose passes spill at 64.
+template <int Z1>
+__host__ __device__ constexpr int zy_blocks() { return Z1 > 8 ? 3 : 4; }
 
 // z and y twiddles from the table into shared memory (they are contiguous in both)
 __device__ __forceinline__ void copy_tw(float2* dst, const float2* __restrict__ src, uint32_t n) {
@@ -138,10 +160,10 @@ struct RowGroup {
 };
 
 // ---------------------------------------------------------------- forward: z (R2C) then y
-template <int Z1, int Z2, int R1, int R2>
-__global__ void __launch_bounds__(256, (Z1 > 8 ? 3 : 4)) plane_zy_fwd(const float* __restrict__ mr, float2* __restrict__ yk,
+template <int Z1, int Z2, int R1, int R2, int CLUSTER>
+__global__ void __launch_bounds__(256, zy_blocks<Z1>()) plane_zy_fwd(const float* __restrict__ mr, float2* __restrict__ yk,
                                                        const PlaneArgs A) {
-    using G = ZYGeom<Z1, Z2, R1, R2>;
+    using G = ZYGeom<Z1, Z2, R1, R2, CLUSTER>;
     constexpr uint32_t N = G::N, KZ = G::KZ, TY = G::TY, LD = G::LD, M1 = G::M1;
     constexpr uint32_t CL = G::CL, HY = G::HY, LDZ = G::LDZ, HK = G::HK, KPB = G::KPB;
     constexpr bool WLZ = rows_warp_local<Z1, Z2>();    // z rows warp-local
@@ -176,7 +198,7 @@ __global__ void __launch_bounds__(256, (Z1 > 8 ? 3 : 4)) plane_zy_fwd(const floa
         // X_k and X_{N-k} from the same two values Z_k, Z_{N-k}
         constexpr uint32_t NH = N / 2 + 1;
         auto split = [&](uint32_t r, uint32_t k) {
-            const float2 zk = scr[r * LD + (k & (N - 1))], zm = scr[r * LD + ((N - k) & (N - 1))];
+            const float2 zk = scr[r * LD + mod_n<N>(k)], zm = scr[r * LD + mod_n<N>(N - k)];
             float2* zc = Zs + (y0 + r - ry0);
             zc[k * LDZ] = r2c_split(zk, zm, ws[k]);
             if (k != N / 2) zc[(N - k) * LDZ] = r2c_split(zm, zk, ws[N - k]);
@@ -257,7 +279,7 @@ __global__ void __launch_bounds__(256, (Z1 > 8 ? 3 : 4)) plane_zy_fwd(const floa
             group_sync<WLY>();
             if (!WLY || threadIdx.x < 32)
                 for (uint32_t ky = threadIdx.x; ky < M1; ky += WLY ? 32u : blockDim.x) {
-                    const float2 a = cpk[ky], b = cpk[(M1 - ky) & (M1 - 1)];
+                    const float2 a = cpk[ky], b = cpk[mod_n<M1>(M1 - ky)];
                     yk[yk_index(A, KZ, c, 0, xl, ky)] = make_float2(0.5f * (a.x + b.x), 0.5f * (a.y - b.y));
                     yk[yk_index(A, KZ, c, N, xl, ky)] = make_float2(0.5f * (a.y + b.y), -0.5f * (a.x - b.x));
                 }
@@ -442,12 +464,10 @@ __global__ void __launch_bounds__(PT * R1, CPLX ? 1 : 3) plane_x_conv(float2* __
 }
 
 // ---------------------------------------------------------------- inverse: y then z (C2R)
-// 4 blocks per SM (64 registers, no spill) where the z rows are at most 64 points (8 × 8), 3
-// for the longer rows, whose passes spill at 64; like the forward kernel.
-template <int Z1, int Z2, int R1, int R2>
-__global__ void __launch_bounds__(256, (Z1 > 8 ? 3 : 4)) plane_yz_inv(const float2* __restrict__ yk, float* __restrict__ hr,
+template <int Z1, int Z2, int R1, int R2, int CLUSTER>
+__global__ void __launch_bounds__(256, zy_blocks<Z1>()) plane_yz_inv(const float2* __restrict__ yk, float* __restrict__ hr,
                                                        const PlaneArgs A) {
-    using G = ZYGeom<Z1, Z2, R1, R2>;
+    using G = ZYGeom<Z1, Z2, R1, R2, CLUSTER>;
     constexpr uint32_t N = G::N, KZ = G::KZ, TY = G::TY, LD = G::LD, M1 = G::M1;
     constexpr uint32_t CL = G::CL, HY = G::HY, LDZ = G::LDZ, HK = G::HK, KPB = G::KPB;
     constexpr bool WLZ = rows_warp_local<Z1, Z2>();
@@ -570,9 +590,12 @@ __global__ void __launch_bounds__(256, (Z1 > 8 ? 3 : 4)) plane_yz_inv(const floa
 
 // ---------------------------------------------------------------- N_k in the tiled layout
 // From the FP64 half spectrum z[q][x][y][kz] (cuFFT D2Z of N_r) to
-// nkt[kz][tile][q][kx][j] (real: float, kx < nkx; complex: float2, kx < m0), ky = tile T + j.
+// nkt[kz][tile][q][kx][j] (real: float, kx < nkx; complex: float2, kx < m0), ky = tile T + j,
+// times 1/P, the scale of the unnormalised transforms: in FP64 before the one rounding, so that a
+// mesh that is not a power of two gives the field no rounded scale factor (a relative error common
+// to every spin and step, which adds up coherently).
 __global__ void nk_tile_real(size_t Pk, uint32_t nkx, uint32_t m1, uint32_t Kz, uint32_t T,
-                             const double2* __restrict__ z, float* __restrict__ out, size_t total) {
+                             const double2* __restrict__ z, double scale, float* __restrict__ out, size_t total) {
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= total) return;
     const uint32_t j = (uint32_t)(e % T);
@@ -582,11 +605,11 @@ __global__ void nk_tile_real(size_t Pk, uint32_t nkx, uint32_t m1, uint32_t Kz, 
     const uint32_t tile = (uint32_t)(rest % (m1 / T));
     const uint32_t kz = (uint32_t)(rest / (m1 / T));
     const uint32_t ky = tile * T + j;
-    out[e] = (float)z[(size_t)q * Pk + ((size_t)kx * m1 + ky) * Kz + kz].x;
+    out[e] = (float)(z[(size_t)q * Pk + ((size_t)kx * m1 + ky) * Kz + kz].x * scale);
 }
 
 __global__ void nk_tile_cplx(size_t Pk, uint32_t m0, uint32_t m1, uint32_t Kz, uint32_t T,
-                             const double2* __restrict__ z, float2* __restrict__ out) {
+                             const double2* __restrict__ z, double scale, float2* __restrict__ out) {
     const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= Pk * 9) return;
     const uint32_t j = (uint32_t)(e % T);
@@ -597,7 +620,7 @@ __global__ void nk_tile_cplx(size_t Pk, uint32_t m0, uint32_t m1, uint32_t Kz, u
     const uint32_t kz = (uint32_t)(rest / (m1 / T));
     const uint32_t ky = tile * T + j;
     const double2 v = z[(size_t)q * Pk + ((size_t)kx * m1 + ky) * Kz + kz];
-    out[e] = make_float2((float)v.x, (float)v.y);
+    out[e] = make_float2((float)(v.x * scale), (float)(v.y * scale));
 }
 
 // Largest |N(kx) - N(m0-kx)| and |N(kx) + N(m0-kx)| (real parts) of each of the 6 components:
@@ -629,31 +652,62 @@ __global__ void nk_parity_x(size_t Pk, uint32_t m0, uint32_t m1, uint32_t Kz, co
     }
 }
 
-// Twiddle table of the plane kernels, rounded from double precision: exp(-2 pi i j / N) (j < N),
-// exp(-i pi k / N) (k <= N), exp(-2 pi i j / m1) (j < m1), exp(-2 pi i j / m0) (j < m0).
-__global__ void tw_table_k(uint32_t N, uint32_t m1, uint32_t m0, float2* __restrict__ t) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t n1 = 2 * N + 1, n2 = n1 + m1, n3 = n2 + m0;
-    if (i >= n3) return;
-    double a;
-    if (i < N) a = -2.0 * (double)i / (double)N;
-    else if (i < n1) a = -(double)(i - N) / (double)N;
-    else if (i < n2) a = -2.0 * (double)(i - n1) / (double)m1;
-    else a = -2.0 * (double)(i - n2) / (double)m0;
-    double sn, cs;
-    sincospi(a, &sn, &cs);
-    t[i] = make_float2((float)cs, (float)sn);
+// N_r re-embedded on another mesh: the displacements |d_a| < b_a between spins of a box of b
+// points, from index d mod m of the caller's mesh to d mod M of this one; the rest is zero (set
+// before).
+__global__ void embed_nr_k(uint3 b, uint3 m, uint3 M, const double* __restrict__ in, double* __restrict__ out) {
+    const uint32_t wx = 2 * b.x - 1, wy = 2 * b.y - 1, wz = 2 * b.z - 1;
+    const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= (size_t)wx * wy * wz) return;
+    const int dz = (int)(e % wz) - (int)(b.z - 1), dy = (int)(e / wz % wy) - (int)(b.y - 1);
+    const int dx = (int)(e / wz / wy) - (int)(b.x - 1);
+    auto at = [&](uint3 q) {
+        const uint32_t x = dx < 0 ? q.x + dx : dx, y = dy < 0 ? q.y + dy : dy, z = dz < 0 ? q.z + dz : dz;
+        return ((size_t)x * q.y + y) * q.z + z;
+    };
+    const size_t i = at(m), o = at(M), P = (size_t)m.x * m.y * m.z, Q = (size_t)M.x * M.y * M.z;
+    for (int c = 0; c < 9; c++) out[c * Q + o] = in[c * P + i];
 }
 
-uint32_t ilog2(uint32_t v) {
-    uint32_t l = 0;
-    while ((1u << l) < v) l++;
-    return l;
+// exp(-2 pi i j / n), exact at the multiples of an eighth turn up to the last bit of a double.
+void unit_root(uint32_t j, uint32_t n, double* c, double* s) {
+    const uint32_t oct = (uint32_t)((uint64_t)8 * j / n), rem = (uint32_t)((uint64_t)8 * j % n);   // angle / (pi / 4)
+    const double a = 0.78539816339744830962 * ((oct & 1) ? (double)(n - rem) : (double)rem) / n;
+    const double x = rem == 0 && !(oct & 1) ? 1.0 : cos(a), y = rem == 0 && !(oct & 1) ? 0.0 : sin(a);
+    static const int swap[8] = {0, 1, 1, 0, 0, 1, 1, 0}, nc[8] = {0, 0, 1, 1, 1, 1, 0, 0}, ns[8] = {0, 0, 0, 0, 1, 1, 1, 1};
+    const double cc = swap[oct & 7] ? y : x, ss = swap[oct & 7] ? x : y;
+    *c = nc[oct & 7] ? -cc : cc;
+    *s = ns[oct & 7] ? ss : -ss;
+}
+
+// count roots exp(-2 pi i j / n), j = 0, 1, ..., in single precision, of unit length on average: each
+// component takes one of the two floats around it, the pair whose length brings the running sum
+// of the lengths' errors closest to zero (nearest rounding leaves short axes with a mean of up to
+// 2e-8, which scales the whole field by that much at every step).
+void add_roots(std::vector<float2>& t, uint32_t count, uint32_t n) {
+    double sum = 0.0;
+    for (uint32_t j = 0; j < count; j++) {
+        double v[2];
+        unit_root(j % n, n, &v[0], &v[1]);
+        float best[2] = {(float)v[0], (float)v[1]};
+        double berr = 1e30;
+        for (int k = 0; k < 4; k++) {
+            float f[2];
+            for (int a = 0; a < 2; a++) {
+                f[a] = (float)v[a];
+                if ((k >> a & 1) && (double)f[a] != v[a]) f[a] = nextafterf(f[a], (double)f[a] < v[a] ? 2.0f : -2.0f);
+            }
+            const double err = sqrt((double)f[0] * f[0] + (double)f[1] * f[1]) - 1.0;
+            if (fabs(sum + err) < fabs(berr)) { berr = sum + err; best[0] = f[0]; best[1] = f[1]; }
+        }
+        sum = berr;
+        t.push_back(make_float2(best[0], best[1]));
+    }
 }
 
 PlaneArgs plane_args(const LongRange& L) {
     PlaneArgs A{};
-    const uint32_t m1 = L.mesh[1], N = L.mesh[2] / 2, Kz = N + 1;
+    const uint32_t m1 = L.mesh[1], N = L.mesh[2] / 2;
     const int z1 = split_r1((int)N), z2 = split_r2((int)N);
     const uint32_t TY = 256 / (uint32_t)std::max(z1, z2);
     const uint32_t LD = fft2pass_pitch(N, (uint32_t)z1, (uint32_t)z2);
@@ -664,8 +718,9 @@ PlaneArgs plane_args(const LongRange& L) {
     A.bx = L.box1[0] - L.box0[0] + 1;
     A.by = L.box1[1] - L.box0[1] + 1;
     A.ntile = m1 / PT;
-    const uint32_t CL = zy_cl(m1), hk = N / CL;       // y-pass slots per block
     const int r1 = split_r1((int)m1), r2 = split_r2((int)m1);
+    A.cl = zy_cl(N, m1, (uint32_t)r1, 3 * A.bx);
+    const uint32_t hk = N / A.cl;                      // y-pass slots per block
     const uint32_t kzmax = 256 / (uint32_t)std::max(r1, r2);
     const uint32_t rounds = (hk + kzmax - 1) / kzmax;
     A.kzb = (hk + rounds - 1) / rounds;                // equal rounds of at most kzmax kz
@@ -680,7 +735,7 @@ PlaneArgs plane_args(const LongRange& L) {
 }
 
 size_t zy_smem(const LongRange& L, const PlaneArgs& A) {
-    const uint32_t N = L.mesh[2] / 2, ldz = zy_hy(L.mesh[1]) | 1u;
+    const uint32_t N = L.mesh[2] / 2, ldz = (L.mesh[1] / (2 * A.cl)) | 1u;
     return sizeof(float2) * ((size_t)(N + 1) * ldz + A.scr + 2 * N + 1 + L.mesh[1]);
 }
 
@@ -696,50 +751,100 @@ cudaError_t set_smem(K kern, size_t bytes) {
     return raise_smem_limit(reinterpret_cast<const void*>(kern), bytes);
 }
 
-// z split x y split instantiations: z N in {4..256}, y mesh in {8..256}
+// z split x y split instantiations: z N in {4..256, 24, 48, 96}, y mesh in {8..256, 48, 96, 192}.
 #define ASD_ZY_CASES(M, Z1, Z2)                                                                           \
     switch (M) {                                                                                          \
     case 8: ASD_ZY_CALL(Z1, Z2, 4, 2) break;                                                              \
     case 16: ASD_ZY_CALL(Z1, Z2, 4, 4) break;                                                             \
     case 32: ASD_ZY_CALL(Z1, Z2, 8, 4) break;                                                             \
+    case 48: ASD_ZY_CALL(Z1, Z2, 8, 6) break;                                                             \
     case 64: ASD_ZY_CALL(Z1, Z2, 8, 8) break;                                                             \
+    case 96: ASD_ZY_CALL(Z1, Z2, 16, 6) break;                                                            \
     case 128: ASD_ZY_CALL(Z1, Z2, 16, 8) break;                                                           \
+    case 192: ASD_ZY_CALL(Z1, Z2, 16, 12) break;                                                          \
     case 256: ASD_ZY_CALL(Z1, Z2, 16, 16) break;                                                          \
     default: return cudaErrorInvalidValue;                                                                \
     }
 
+// The z sizes are compiled in four translation units of this file (ASD_ZY_PART 0..3), beside the
+// one with the rest.
+#if ASD_ZY_PART == 0
+#define ASD_ZY_RUN run_zy_part0
 #define ASD_Z_CASES(N, M)                                                                                 \
     switch (N) {                                                                                          \
     case 4: ASD_ZY_CASES(M, 2, 2) break;                                                                  \
     case 8: ASD_ZY_CASES(M, 4, 2) break;                                                                  \
     case 16: ASD_ZY_CASES(M, 4, 4) break;                                                                 \
+    default: return cudaErrorInvalidValue;                                                                \
+    }
+#elif ASD_ZY_PART == 1
+#define ASD_ZY_RUN run_zy_part1
+#define ASD_Z_CASES(N, M)                                                                                 \
+    switch (N) {                                                                                          \
+    case 24: ASD_ZY_CASES(M, 8, 3) break;                                                                 \
     case 32: ASD_ZY_CASES(M, 8, 4) break;                                                                 \
+    default: return cudaErrorInvalidValue;                                                                \
+    }
+#elif ASD_ZY_PART == 2
+#define ASD_ZY_RUN run_zy_part2
+#define ASD_Z_CASES(N, M)                                                                                 \
+    switch (N) {                                                                                          \
+    case 48: ASD_ZY_CASES(M, 8, 6) break;                                                                 \
     case 64: ASD_ZY_CASES(M, 8, 8) break;                                                                 \
+    default: return cudaErrorInvalidValue;                                                                \
+    }
+#elif ASD_ZY_PART == 3
+#define ASD_ZY_RUN run_zy_part3
+#define ASD_Z_CASES(N, M)                                                                                 \
+    switch (N) {                                                                                          \
+    case 96: ASD_ZY_CASES(M, 16, 6) break;                                                                \
     case 128: ASD_ZY_CASES(M, 16, 8) break;                                                               \
     case 256: ASD_ZY_CASES(M, 16, 16) break;                                                              \
     default: return cudaErrorInvalidValue;                                                                \
     }
+#endif
 
-cudaError_t run_zy(const LongRange& L, const PlaneArgs& A, bool inverse, cudaStream_t st, bool pdl) {
-    const size_t sm = zy_smem(L, A);
-    const uint32_t CL = zy_cl(L.mesh[1]);
-    const dim3 grid(A.bx * CL, 3);
-    const float* mr = L.r;
-    float* hr = L.r + 3 * L.P;
-    float2* yk = L.yk;
-    const float2* ykc = L.yk;
+#ifdef ASD_ZY_PART
+template <int Z1, int Z2, int R1, int R2, int CL>
+cudaError_t run_zy_k(const LongRange& L, const PlaneArgs& A, bool inverse, cudaStream_t st, bool pdl) {
+    if constexpr (!zy_cl_used(Z1 * Z2, R1 * R2, R1, CL)) {
+        return cudaErrorInvalidValue;
+    } else {
+        const size_t sm = zy_smem(L, A);
+        const dim3 grid(A.bx * CL, 3);
+        const float2* ykc = L.yk;
+        const float* mr = L.r;
+        float* hr = L.r + 3 * L.P;
+        cudaError_t e;
+        if (inverse) {
+            if ((e = set_smem(plane_yz_inv<Z1, Z2, R1, R2, CL>, sm)) != cudaSuccess) return e;
+            e = launch_step_kernel(plane_yz_inv<Z1, Z2, R1, R2, CL>, grid, dim3(256), sm, st, CL, pdl, ykc, hr, A);
+        } else {
+            if ((e = set_smem(plane_zy_fwd<Z1, Z2, R1, R2, CL>, sm)) != cudaSuccess) return e;
+            e = launch_step_kernel(plane_zy_fwd<Z1, Z2, R1, R2, CL>, grid, dim3(256), sm, st, CL, pdl, mr, L.yk, A);
+        }
+        return e;
+    }
+}
+}  // namespace
+
+cudaError_t ASD_ZY_RUN(const LongRange& L, bool inverse, cudaStream_t st, bool pdl) {
+    const PlaneArgs A = plane_args(L);
     cudaError_t e = cudaSuccess;
 #define ASD_ZY_CALL(Z1, Z2, R1, R2)                                                                       \
-    if (inverse) {                                                                                        \
-        if ((e = set_smem(plane_yz_inv<Z1, Z2, R1, R2>, sm)) != cudaSuccess) return e;                    \
-        e = launch_step_kernel(plane_yz_inv<Z1, Z2, R1, R2>, grid, dim3(256), sm, st, CL, pdl, ykc, hr, A); \
-    } else {                                                                                              \
-        if ((e = set_smem(plane_zy_fwd<Z1, Z2, R1, R2>, sm)) != cudaSuccess) return e;                    \
-        e = launch_step_kernel(plane_zy_fwd<Z1, Z2, R1, R2>, grid, dim3(256), sm, st, CL, pdl, mr, yk, A);  \
-    }
+    e = A.cl == 1 ? run_zy_k<Z1, Z2, R1, R2, 1>(L, A, inverse, st, pdl)                                    \
+        : A.cl == 2 ? run_zy_k<Z1, Z2, R1, R2, 2>(L, A, inverse, st, pdl)                                  \
+                    : run_zy_k<Z1, Z2, R1, R2, 4>(L, A, inverse, st, pdl);
     ASD_Z_CASES(L.mesh[2] / 2, L.mesh[1])
 #undef ASD_ZY_CALL
     return e != cudaSuccess ? e : cudaGetLastError();
+}
+#else
+
+cudaError_t run_zy(const LongRange& L, bool inverse, cudaStream_t st, bool pdl) {
+    const uint32_t N = L.mesh[2] / 2;
+    return N <= 16 ? run_zy_part0(L, inverse, st, pdl) : N <= 32 ? run_zy_part1(L, inverse, st, pdl)
+           : N <= 64 ? run_zy_part2(L, inverse, st, pdl) : run_zy_part3(L, inverse, st, pdl);
 }
 
 template <int R1, int R2, bool CPLX>
@@ -772,27 +877,49 @@ cudaError_t run_xconv(const LongRange& L, const PlaneArgs& A, bool cplx, cudaStr
     case 64: return run_xconv_t<8, 8>(L, A, cplx, st, pdl);
     case 128: return run_xconv_t<16, 8>(L, A, cplx, st, pdl);
     case 256: return run_xconv_t<16, 16>(L, A, cplx, st, pdl);
+    case 24: return run_xconv_t<8, 3>(L, A, cplx, st, pdl);
+    case 48: return run_xconv_t<8, 6>(L, A, cplx, st, pdl);
+    case 96: return run_xconv_t<16, 6>(L, A, cplx, st, pdl);
+    case 192: return run_xconv_t<16, 12>(L, A, cplx, st, pdl);
     default: return cudaErrorInvalidValue;
     }
 }
 
 }  // namespace
 
-// The plane path applies when every mesh axis is a power of two (x 4..256, y 8..256, z 8..512:
-// the register transforms' sizes), the spins' box spans at most half the mesh along x and y and
-// its z pairs fit in half a row (so every forward pass skips the zero half of its input and
-// every inverse pass forms only the box half of its output), and the shared memory fits.
+// Axis lengths of the plane kernels' transforms, ascending: powers of two and 3 x powers of two
+// (from 48 on, where the step from one power of two to the next costs time).
+constexpr uint32_t X_LEN[] = {4, 8, 16, 24, 32, 48, 64, 96, 128, 192, 256};
+constexpr uint32_t Y_LEN[] = {8, 16, 32, 48, 64, 96, 128, 192, 256};
+constexpr uint32_t Z_LEN[] = {8, 16, 32, 48, 64, 96, 128, 192, 256, 512};
+
+template <size_t K>
+bool has_len(const uint32_t (&len)[K], uint32_t v) { return std::find(len, len + K, v) != len + K; }
+template <size_t K>
+uint32_t len_from(const uint32_t (&len)[K], uint32_t least) {
+    const uint32_t* p = std::lower_bound(len, len + K, least);
+    return p == len + K ? 0 : *p;
+}
+
+// The plane path applies when every mesh axis has one of the kernels' lengths, the spins' box
+// spans at most half the mesh along x and y and its z pairs fit in half a row (so every forward
+// pass skips the zero half of its input and every inverse pass forms only the box half of its
+// output), and the shared memory fits.
 bool plane_path_fits(const LongRange& L, bool cplx) {
-    auto p2 = [](uint32_t v) { return v >= 2 && (v & (v - 1)) == 0; };
-    if (!p2(L.mesh[0]) || !p2(L.mesh[1]) || !p2(L.mesh[2])) return false;
-    if (L.mesh[0] < 4 || L.mesh[0] > 256 || L.mesh[1] < 8 || L.mesh[1] > 256 || L.mesh[2] < 8 || L.mesh[2] > 512)
-        return false;
+    if (!has_len(X_LEN, L.mesh[0]) || !has_len(Y_LEN, L.mesh[1]) || !has_len(Z_LEN, L.mesh[2])) return false;
     LongRange t = L;
     t.nk_nkx = L.mesh[0];                              // the larger N_k tile bounds the shared memory
     const PlaneArgs A = plane_args(t);
     const uint32_t N = L.mesh[2] / 2;
     if (2 * A.bx > L.mesh[0] || 2 * A.by > L.mesh[1] || 2 * A.nz > N) return false;
     return zy_smem(L, A) <= 200 * 1024 && xconv_smem(A, cplx) <= 220 * 1024;
+}
+
+// The shortest mesh of the plane kernels that holds twice the box (0 in an axis: none does).
+void plane_mesh_for(const uint32_t box[3], uint32_t mesh[3]) {
+    mesh[0] = len_from(X_LEN, 2 * box[0]);
+    mesh[1] = len_from(Y_LEN, 2 * box[1]);
+    mesh[2] = len_from(Z_LEN, 2 * box[2]);
 }
 
 size_t plane_spectrum_elems(const LongRange& L) {
@@ -807,6 +934,7 @@ cudaError_t build_nk_tiles(asd_handle* h, const double2* z, uint32_t ncomp, bool
     LongRange& L = h->lr;
     const uint32_t Kz = L.mesh[2] / 2 + 1;
     const size_t Pk = (size_t)L.mesh[0] * L.mesh[1] * Kz;
+    const double scale = 1.0 / (double)L.P;
     cudaError_t e;
     if (!cplx) {
         unsigned long long* dev = nullptr;
@@ -835,7 +963,7 @@ cudaError_t build_nk_tiles(asd_handle* h, const double2* z, uint32_t ncomp, bool
         const size_t total = (size_t)6 * L.nk_nkx * L.mesh[1] * Kz;
         float* t = nullptr;
         if ((e = cudaMalloc(&t, sizeof(float) * total)) != cudaSuccess) return e;
-        nk_tile_real<<<nbk(total, 256), 256, 0, h->stream>>>(Pk, L.nk_nkx, L.mesh[1], Kz, PT, z, t, total);
+        nk_tile_real<<<nbk(total, 256), 256, 0, h->stream>>>(Pk, L.nk_nkx, L.mesh[1], Kz, PT, z, scale, t, total);
         L.nkt = t;
     } else {
         float2* t = nullptr;
@@ -843,9 +971,20 @@ cudaError_t build_nk_tiles(asd_handle* h, const double2* z, uint32_t ncomp, bool
         (void)ncomp;
         L.nk_nkx = L.mesh[0];
         L.nk_odd = 0;
-        nk_tile_cplx<<<nbk(9 * Pk, 256), 256, 0, h->stream>>>(Pk, L.mesh[0], L.mesh[1], Kz, PT, z, t);
+        nk_tile_cplx<<<nbk(9 * Pk, 256), 256, 0, h->stream>>>(Pk, L.mesh[0], L.mesh[1], Kz, PT, z, scale, t);
         L.nkt = t;
     }
+    return cudaGetLastError();
+}
+
+cudaError_t embed_nr(asd_handle* h, const uint32_t box[3], const uint32_t from[3], const uint32_t to[3],
+                     const double* d_in, double* d_out) {
+    const size_t n = (size_t)(2 * box[0] - 1) * (2 * box[1] - 1) * (2 * box[2] - 1);
+    const cudaError_t e = cudaMemsetAsync(d_out, 0, sizeof(double) * 9 * to[0] * to[1] * to[2], h->stream);
+    if (e != cudaSuccess) return e;
+    embed_nr_k<<<nbk(n, 256), 256, 0, h->stream>>>(make_uint3(box[0], box[1], box[2]),
+                                                   make_uint3(from[0], from[1], from[2]),
+                                                   make_uint3(to[0], to[1], to[2]), d_in, d_out);
     return cudaGetLastError();
 }
 
@@ -858,7 +997,13 @@ cudaError_t build_plane_twiddles(asd_handle* h) {
     if (e != cudaSuccess) return e;
     if ((e = cudaMalloc(&L.xq, 2 * sizeof(uint32_t))) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(L.xq, 0, 2 * sizeof(uint32_t), h->stream)) != cudaSuccess) return e;
-    tw_table_k<<<nbk(n, 256), 256, 0, h->stream>>>(N, L.mesh[1], L.mesh[0], L.twt);
+    std::vector<float2> t;
+    add_roots(t, N, N);                                // z
+    add_roots(t, N + 1, 2 * N);                        // z split: exp(-i pi k / N), k <= N
+    add_roots(t, L.mesh[1], L.mesh[1]);
+    add_roots(t, L.mesh[0], L.mesh[0]);
+    if ((e = cudaMemcpyAsync(L.twt, t.data(), sizeof(float2) * n, cudaMemcpyHostToDevice, h->stream)) != cudaSuccess) return e;
+    if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return e;
     return cudaGetLastError();
 }
 
@@ -878,16 +1023,18 @@ cudaError_t launch_lr_planes(asd_handle* h) {
     cudaError_t e;
     timer_begin(h);
     const bool pdl = step_pdl(h);
-    if ((e = run_zy(L, A, false, h->stream, pdl)) != cudaSuccess) return e;
+    if ((e = run_zy(L, false, h->stream, pdl)) != cudaSuccess) return e;
     timer_end(h, "plane_zy_fwd (z R2C + y FFT)", rows + spec);
     timer_begin(h);
     if ((e = run_xconv(L, A, cplx, h->stream, pdl)) != cudaSuccess) return e;
     timer_end(h, "plane_x_conv (x FFT, N_k product, inverse x FFT)", 2.0 * spec + nkb);
     timer_begin(h);
-    if ((e = run_zy(L, A, true, h->stream, pdl)) != cudaSuccess) return e;
+    if ((e = run_zy(L, true, h->stream, pdl)) != cudaSuccess) return e;
     timer_end(h, "plane_yz_inv (inverse y FFT + z C2R)", spec + rows);
     h->launches += 3;
     return cudaSuccess;
 }
+
+#endif  // ASD_ZY_PART
 
 }  // namespace asd

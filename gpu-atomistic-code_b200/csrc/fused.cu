@@ -584,7 +584,7 @@ cudaError_t fused_step_t(asd_handle* h, uint32_t rel) {
     const uint32_t upd = h->p.update ? h->p.update : 1;
     LongRange& L = h->lr;
     LrArgs none{};
-    none.P = L.P; none.idx = L.mesh_idx; none.w = L.w; none.inv_p = L.P ? 1.0f / (float)L.P : 0.f;
+    none.P = L.P; none.idx = L.mesh_idx; none.w = L.w; none.inv_p = L.scale();
     cudaError_t e;
     cudaError_t e0;
     if (h->d_ttm && (e0 = launch_ttm_step(h, h->d_step, rel)) != cudaSuccess) return e0;

@@ -118,6 +118,8 @@ struct LongRange {
     uint32_t nk_nkx = 0, nk_odd = 0;   // kx rows of the tiled N_k and its odd components (bits)
     float2* yk = nullptr;
     void* nkt = nullptr;
+    // factor of the gathered field: the plane kernels' N_k carries 1/P, cuFFT's transforms do not
+    float scale() const { return planes || !P ? 1.0f : 1.0f / (float)P; }
     float2* twt = nullptr;          // twiddle table of the plane kernels
     uint32_t* xq = nullptr;           // x-pass item counters: next item, finished blocks
     // FP64 plain: complex padded arrays [3][P] and full complex N_k [9][P]
@@ -283,8 +285,16 @@ const void* det_here_kernel();
 cudaError_t launch_lr_eval_f32(asd_handle* h);
 cudaError_t launch_lr_scatter(asd_handle* h);
 cudaError_t launch_lr_planes(asd_handle* h);
+// the z/y plane kernels (inverse or forward) of z rows of up to 16, 32, 64 and 256 points
+cudaError_t run_zy_part0(const LongRange& L, bool inverse, cudaStream_t st, bool pdl);
+cudaError_t run_zy_part1(const LongRange& L, bool inverse, cudaStream_t st, bool pdl);
+cudaError_t run_zy_part2(const LongRange& L, bool inverse, cudaStream_t st, bool pdl);
+cudaError_t run_zy_part3(const LongRange& L, bool inverse, cudaStream_t st, bool pdl);
 cudaError_t build_plane_twiddles(asd_handle* h);
 bool plane_path_fits(const LongRange& L, bool cplx);
+void plane_mesh_for(const uint32_t box[3], uint32_t mesh[3]);
+cudaError_t embed_nr(asd_handle* h, const uint32_t box[3], const uint32_t from[3], const uint32_t to[3],
+                     const double* d_in, double* d_out);
 size_t plane_spectrum_elems(const LongRange& L);
 cudaError_t build_nk_tiles(asd_handle* h, const double2* z, uint32_t ncomp, bool cplx);
 cudaError_t launch_lr_eval_plain(asd_handle* h, const double* s, double* out, bool overwrite_with_demag);

@@ -364,7 +364,7 @@ cudaError_t field_t(asd_handle* h, double* out) {
         }
         hr = h->lr.r + 3 * h->lr.P;
     }
-    const float inv_p = h->lr.P ? 1.0f / (float)h->lr.P : 0.f;
+    const float inv_p = h->lr.scale();
     const unsigned g = nb(h->n, 256);
     const size_t cs = sizeof(R) * (h->full ? table_stride<true>() : table_stride<false>());
     if (h->dexch == ASD_EXCH_CSR) {

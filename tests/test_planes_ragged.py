@@ -1,0 +1,82 @@
+"""Long-range field on meshes whose axes are not powers of two: the library moves N_r to the
+shortest mesh of the plane kernels' lengths (powers of two and 3 x powers of two) that holds twice
+the box.  Against the FP64 direct-sum oracle on the caller's mesh; each
+new length is reached at an edge of its range.  Tolerances as in the power-of-two tests: FP32
+1e-5, fused FP64 with the FP32 transform 1e-8."""
+import numpy as np
+import pytest
+
+import asd_b200 as A
+import asd_lattice as LT
+from helpers import maxdiff
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+PLANES = "long-range: plane kernels"
+
+
+FP32 = (A.FP32, A.FLAG_COMPENSATED, 1e-5)
+FUSED64 = (A.FP64_FUSED, 0, 1e-8)
+
+
+def check(s, steps, forms=(FP32, FUSED64)):
+    S0 = LT.random_spins(s.nspins, 0)
+    o = O.Oracle(s)
+    o.set_spins(S0)
+    o.step(steps)
+    for prec, flags, tol in forms:
+        with A.Handle(A.RunParams(precision=prec, flags=flags), s) as h:
+            assert PLANES in h.tuning(), h.tuning()
+            h.set_spins(S0)
+            h.step(steps)
+            g = h.get_spins()
+        assert maxdiff(g, o.spins()) <= tol, (prec, maxdiff(g, o.spins()))
+
+
+# x, y, z lengths the box leads to in the comments
+@pytest.mark.parametrize("L", [(9, 11, 1),       # 24, 32, 8 (caller's mesh z: 2)
+                               (12, 20, 3),      # 24, 48, 8
+                               (20, 3, 23),      # 48, 8, 48
+                               (2, 37, 33),      # 4, 96, 96
+                               (40, 5, 17),      # 96, 16, 48
+                               (67, 3, 5),       # 192, 8, 16
+                               (1, 66, 70),      # 4, 192, 192: one row, clusters of 4
+                               (100, 33, 1),     # 256, 96, 8: 300 rows of one block
+                               (87, 9, 3)])      # 192, 32, 8
+def test_ragged_dipole_matches_oracle(gpu, L):
+    check(LT.sc_ferromagnet(L, pbc=(0, 0, 0), dipole=True), 10)
+
+
+def test_ragged_box_away_from_origin(gpu):
+    s = LT.sc_ferromagnet((5, 6, 3), pbc=(0, 0, 0), dipole=True)
+    s.nr, s.mesh = LT.dipole_nr((9, 7, 5))
+    s.mesh_xyz = (LT.sc_mesh_xyz((5, 6, 3)) + np.array((11, 3, 6), dtype=np.uint32)).astype(np.uint32)
+    check(s, 20)
+
+
+def test_ragged_general_interaction_matrix(gpu):
+    """Neither symmetric nor even: 9 complex N_k components on the new mesh."""
+    s = LT.sc_ferromagnet((5, 9, 7), pbc=(0, 0, 0), dipole=True)
+    rng = np.random.default_rng(7)
+    s.nr = s.nr + rng.uniform(-0.05, 0.05, s.nr.shape) * np.abs(s.nr).max()
+    check(s, 20)
+
+
+def test_ragged_fft_exchange_mode(gpu):
+    """The whole field from N_k (FP32 form, as for the power-of-two meshes: the fused FP64 form's
+    1e-8 is the dipole's, a thousandth of the field)."""
+    check(LT.sc_fft((6, 5, 7)), 40, (FP32,))
+
+
+def test_box_wider_than_the_plane_kernels(gpu):
+    """An axis of more than 128 points has no plane-kernel length: cuFFT runs the caller's mesh."""
+    s = LT.sc_ferromagnet((131, 2, 3), pbc=(0, 0, 0), dipole=True)
+    S0 = LT.random_spins(s.nspins, 0)
+    o = O.Oracle(s)
+    o.set_spins(S0)
+    o.step(10)
+    with A.Handle(A.RunParams(precision=A.FP32, flags=A.FLAG_COMPENSATED), s) as h:
+        assert "cuFFT" in h.tuning(), h.tuning()
+        h.set_spins(S0)
+        h.step(10)
+        assert maxdiff(h.get_spins(), o.spins()) <= 1e-5
