@@ -152,39 +152,39 @@ void build_patterns(asd_handle* h, const std::vector<uint32_t>& xadj, const std:
     uint32_t W = 0;
     for (uint32_t i = 0; i < n; i++) W = std::max(W, xadj[i + 1] - xadj[i]);
     if (W == 0 || (uint64_t)W * n > (uint64_t)sell_entries + sell_entries / 4) return;
-    std::vector<int2> ent;                            // [pattern][W]
+    W += W & 1;
+    std::vector<int32_t> ent;                         // [pattern][W]
     std::vector<uint32_t> plen;                       // its entries before the padding
     std::vector<uint16_t> row(n);
     std::unordered_multimap<uint64_t, uint32_t> seen;  // hash of a pattern -> its number
-    std::vector<int2> cur(W);
+    std::vector<int32_t> cur(W);
     const size_t most = std::min<size_t>(65536, adj.size() / (4 * (size_t)W));
+    auto word = [](uint32_t col, uint32_t i, uint32_t typ) { return (int32_t)(((col - i) << 8) | typ); };
     for (uint32_t i = 0; i < n; i++) {
         const uint32_t len = xadj[i + 1] - xadj[i];
         const uint32_t* col = adj.data() + xadj[i];
         const uint32_t* typ = id.data() + xadj[i];
         auto same = [&](uint32_t p) {
-            const int2* e = ent.data() + (size_t)p * W;
+            const int32_t* e = ent.data() + (size_t)p * W;
             for (uint32_t k = 0; k < len; k++)
-                if ((uint32_t)e[k].x != col[k] - i || (uint32_t)e[k].y != typ[k]) return false;
+                if (e[k] != word(col[k], i, typ[k])) return false;
             return plen[p] == len;
         };
+        for (uint32_t k = 0; k < len; k++)
+            if (std::abs((int64_t)col[k] - (int64_t)i) >= PAT_DELTA) return;
         // a lattice repeats the pattern of one of the last rows nearly always
         uint32_t p = ~0u;
         for (uint32_t back = 1; back <= 4 && back <= i && p == ~0u; back++)
             if (same(row[i - back])) p = row[i - back];
         if (p == ~0u) {
-            for (uint32_t k = 0; k < W; k++)
-                cur[k] = k < len ? make_int2((int)(col[k] - i), (int)typ[k]) : make_int2(0, 0);
+            for (uint32_t k = 0; k < W; k++) cur[k] = k < len ? word(col[k], i, typ[k]) : 0;
             uint64_t hash = 0xcbf29ce484222325ull;     // FNV-1a over the words
-            for (const int2& v : cur) {
-                hash = (hash ^ (uint32_t)v.x) * 0x100000001b3ull;
-                hash = (hash ^ (uint32_t)v.y) * 0x100000001b3ull;
-            }
+            for (const int32_t v : cur) hash = (hash ^ (uint32_t)v) * 0x100000001b3ull;
             const auto range = seen.equal_range(hash);
             for (auto it = range.first; it != range.second && p == ~0u; ++it)
                 if (same(it->second)) p = it->second;
             if (p == ~0u) {
-                p = (uint32_t)(ent.size() / W);
+                p = (uint32_t)plen.size();
                 if (p >= most) return;
                 ent.insert(ent.end(), cur.begin(), cur.end());
                 plen.push_back(len);
@@ -194,13 +194,13 @@ void build_patterns(asd_handle* h, const std::vector<uint32_t>& xadj, const std:
         row[i] = (uint16_t)p;
     }
     h->pat.W = W;
-    h->pat.npat = (uint32_t)(ent.size() / W);
+    h->pat.npat = (uint32_t)plen.size();
     h->pat.row = dupload(row.data(), row.size());
     h->pat.ent = dupload(ent.data(), ent.size());
 }
 
 // CSR (all replicas concatenated) -> SELL-32 device layout.
-void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vector<uint32_t>& adj,
+void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vector<uint32_t>& adj0,
                 const double* val9) {
     const uint32_t n = h->n;
     const bool full = h->full != 0;
@@ -226,9 +226,9 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
         const int nc = full ? 9 : 3;
         const int qmap[9] = {0, 4, 8, 0, 0, 0, 0, 0, 0};
         TensorTable tt(nc);
-        std::vector<uint32_t> id(adj.size());
+        std::vector<uint32_t> id(adj0.size());
         bool ok = true;
-        for (size_t k = 0; k < adj.size() && ok; k++) {
+        for (size_t k = 0; k < adj0.size() && ok; k++) {
             std::array<double, 9> key{};
             for (int q = 0; q < nc; q++) key[q] = value((uint32_t)k, full ? q : qmap[q]);
             const int64_t t = tt.id(key);
@@ -236,6 +236,23 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
         }
         const uint32_t tb = tt.bits();
         if (ok && (uint64_t)n <= (1ull << (32 - tb))) {
+            // full tensors: a row's entries by tensor (RowSum), in the caller's order within one; DIA
+            // input comes in its diagonals' order by tensor already (diag_order)
+            std::vector<uint32_t> col_by;
+            if (full && h->exch == ASD_EXCH_CSR && h->p.precision != ASD_FP64_PLAIN) {
+                col_by = adj0;
+                std::vector<std::pair<uint32_t, uint32_t>> rowv;
+                for (uint32_t r = 0; r < n; r++) {
+                    const uint32_t e0 = xadj[r], e1 = xadj[r + 1];
+                    if (std::is_sorted(id.begin() + e0, id.begin() + e1)) continue;
+                    rowv.clear();
+                    for (uint32_t k = e0; k < e1; k++) rowv.emplace_back(id[k], adj0[k]);
+                    std::stable_sort(rowv.begin(), rowv.end(),
+                                     [](const auto& a, const auto& b) { return a.first < b.first; });
+                    for (uint32_t k = e0; k < e1; k++) { id[k] = rowv[k - e0].first; col_by[k] = rowv[k - e0].second; }
+                }
+            }
+            const std::vector<uint32_t>& adj = col_by.empty() ? adj0 : col_by;
             std::vector<uint32_t> w(E);
             for (uint32_t s = 0; s < ns; s++) {
                 const uint32_t wd = (sp[s + 1] - sp[s]) / 32;
@@ -262,6 +279,7 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
             return;
         }
     }
+    if (h->p.precision == ASD_FP64_PLAIN) return;      // the plain form's own CSR arrays
     if (h->p.precision == ASD_FP32) {
         std::vector<float4> a(E), b(full ? E : 0);
         std::vector<float2> c(full ? E : 0);
@@ -274,7 +292,7 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
                     float v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
                     if (r < n && k < xadj[r + 1] - xadj[r]) {
                         const uint32_t kk = xadj[r] + k;
-                        col = (int)adj[kk];
+                        col = (int)adj0[kk];
                         for (int q = 0; q < 9; q++) v[q] = (float)value(kk, q);
                     }
                     int ci;
@@ -304,13 +322,36 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
                     col[e] = r < n ? (int)r : 0;
                     if (r < n && k < xadj[r + 1] - xadj[r]) {
                         const uint32_t kk = xadj[r] + k;
-                        col[e] = (int)adj[kk];
+                        col[e] = (int)adj0[kk];
                         for (int q = 0; q < nc; q++) v[(size_t)q * E + e] = value(kk, full ? q : qmap3[q]);
                     }
                 }
         }
         h->sell.col = dupload(col.data(), col.size());
         h->sell.val = dupload(v.data(), v.size());
+    }
+}
+
+// The rows of a DIA matrix as CSR, entries in the diagonals' `order`, exact zeros left out.
+template <typename Comp>
+void dia_rows(uint32_t n, uint32_t ndiag, const std::vector<int32_t>& doff, const std::vector<uint32_t>& order,
+              Comp comp, std::vector<uint32_t>& cx, std::vector<uint32_t>& ca, std::vector<double>& cv) {
+    cx.assign((size_t)n + 1, 0);
+    const double* cp[9];
+    for (int q = 0; q < 9; q++) cp[q] = ndiag ? comp(q) : nullptr;
+    for (uint32_t i = 0; i < n; i++) {
+        for (uint32_t d : order) {
+            const int64_t col = (int64_t)i + doff[d];
+            if (col < 0 || col >= (int64_t)n) continue;
+            double v9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+            bool any = false;
+            for (int q = 0; q < 9; q++)
+                if (cp[q]) { v9[q] = cp[q][(size_t)d * n + i]; any |= v9[q] != 0.0; }
+            if (!any) continue;
+            ca.push_back((uint32_t)col);
+            cv.insert(cv.end(), v9, v9 + 9);
+        }
+        cx[i + 1] = (uint32_t)ca.size();
     }
 }
 
@@ -1047,18 +1088,31 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
                 for (int q = 0; q < (p.integrator == ASD_RK4 ? 4 : 6); q++) h->p_k[q] = dalloc<double>(n3);
             if (h->exch == ASD_EXCH_CSR) {
                 h->pex.xadj = dupload(xadj.data(), xadj.size());
-                h->pex.adjncy = dupload(adj.data(), adj.size());
-                std::vector<double> comp(adj.size());
-                for (int q = 0; q < 9; q++) {
-                    for (size_t k = 0; k < adj.size(); k++) comp[k] = val9[9 * k + q];
-                    h->pex.v[q] = dupload(comp.data(), comp.size());
+                build_sell(h, xadj, adj, val9);
+                if (!h->sell.typed) {
+                    h->pex.adjncy = dupload(adj.data(), adj.size());
+                    std::vector<double> comp(adj.size());
+                    for (int q = 0; q < 9; q++) {
+                        for (size_t k = 0; k < adj.size(); k++) comp[k] = val9[9 * k + q];
+                        h->pex.v[q] = dupload(comp.data(), comp.size());
+                    }
                 }
             } else if (h->exch == ASD_EXCH_DIA) {
-                h->pex.ndiag = s0.ndiag;
-                h->pex.off = dupload(doff.data(), doff.size());
-                for (int q = 0; q < 9; q++)
-                    if (dia_comp(q)) h->pex.v[q] = dupload(dia_comp(q), mdia);
+                std::vector<uint32_t> cx, ca;
+                std::vector<double> cv;
+                std::vector<uint32_t> order(s0.ndiag);
+                for (uint32_t d = 0; d < s0.ndiag; d++) order[d] = d;
+                dia_rows(n, s0.ndiag, doff, order, dia_comp, cx, ca, cv);
+                h->pex.xadj = dupload(cx.data(), cx.size());
+                build_sell(h, cx, ca, cv.data());
+                if (!h->sell.typed) {
+                    h->pex.ndiag = s0.ndiag;
+                    h->pex.off = dupload(doff.data(), doff.size());
+                    for (int q = 0; q < 9; q++)
+                        if (dia_comp(q)) h->pex.v[q] = dupload(dia_comp(q), mdia);
+                }
             }
+            h->h_words.clear();                           // (only the fused forms stage words)
             (void)zz_yy;  // applied inside the plain kernels
         } else {
             const size_t bytes = p.precision == ASD_FP32 ? 4 : 8;
@@ -1091,30 +1145,9 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
                 const size_t m = (size_t)s0.ndiag * n;
                 const int nc = h->full ? 9 : 3;
                 const int qmap3[3] = {0, 4, zz_yy ? 4 : 8};
-                {
-                    // active diagonals of every 32-row tile: a periodic lattice has many distinct
-                    // offsets, each row only a few nonzero ones
-                    const uint32_t nt = (n + 31) / 32;
-                    std::vector<uint32_t> tp(nt + 1, 0), td;
-                    const double* comp[9];
-                    for (int q = 0; q < nc; q++) comp[q] = dia_comp(h->full ? q : qmap3[q]);
-                    for (uint32_t w = 0; w < nt; w++) {
-                        const uint32_t r0 = 32 * w, r1 = std::min(n, r0 + 32);
-                        for (uint32_t d = 0; d < s0.ndiag; d++) {
-                            bool any = false;
-                            for (uint32_t r = r0; r < r1 && !any; r++) {
-                                const int64_t col = (int64_t)r + doff[d];
-                                if (col < 0 || col >= (int64_t)n) continue;
-                                for (int q = 0; q < nc && !any; q++) any = comp[q][(size_t)d * n + r] != 0.0;
-                            }
-                            if (any) td.push_back(d);
-                        }
-                        tp[w + 1] = (uint32_t)td.size();
-                    }
-                    h->dia.tile_ptr = dupload(tp.data(), tp.size());
-                    h->dia.tile_diag = dupload(td.data(), std::max<size_t>(td.size(), 1));
-                }
                 bool typed = false;
+                std::vector<uint32_t> diag_order(s0.ndiag);   // the order the gathers take the diagonals in
+                for (uint32_t d = 0; d < s0.ndiag; d++) diag_order[d] = d;
                 if (!(p.flags & ASD_FLAG_STREAMED_EXCHANGE)) {
                     // typed DIA: one id byte per (diagonal, row) into the distinct tensors
                     TensorTable tt(nc);
@@ -1131,6 +1164,19 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
                     if (ok) {
                         h->dia.dtype = dupload(ids.data(), ids.size());
                         h->dia.ntypes = tt.size();
+                        if (h->full) {
+                            // full tensors: the diagonals by their smallest tensor id, so that the
+                            // entries of one tensor follow each other in the rows (RowSum)
+                            std::vector<uint32_t> key(s0.ndiag, 256);
+                            for (uint32_t d = 0; d < s0.ndiag; d++)
+                                for (uint32_t i = 0; i < n; i++) {
+                                    const int64_t col = (int64_t)i + doff[d];
+                                    const uint32_t t = ids[(size_t)d * n + i];
+                                    if (t && t < key[d] && col >= 0 && col < (int64_t)n) key[d] = t;
+                                }
+                            std::stable_sort(diag_order.begin(), diag_order.end(),
+                                             [&](uint32_t a, uint32_t b) { return key[a] < key[b]; });
+                        }
                         if (bytes == 4) { std::vector<float> tf = tt.table<float>(); h->dia.tab_f = dupload(tf.data(), tf.size()); }
                         else { std::vector<double> td = tt.table<double>(); h->dia.tab_d = dupload(td.data(), td.size()); }
                         typed = true;
@@ -1154,27 +1200,35 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
                     }
                     h->dia.vald = dupload(v.data(), v.size());
                 }
-                // the same matrix as SELL-32 for the fused kernels: rows take their entries in
-                // ascending diagonal order, the order the DIA gather sums them in
                 {
-                    std::vector<uint32_t> cx(n + 1, 0), ca;
-                    std::vector<double> cv;
-                    for (uint32_t i = 0; i < n; i++) {
-                        for (uint32_t d = 0; d < s0.ndiag; d++) {
-                            const int64_t col = (int64_t)i + doff[d];
-                            if (col < 0 || col >= (int64_t)n) continue;
-                            double v9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+                    // active diagonals of every 32-row tile: a periodic lattice has many distinct
+                    // offsets, each row only a few nonzero ones
+                    const uint32_t nt = (n + 31) / 32;
+                    std::vector<uint32_t> tp(nt + 1, 0), td;
+                    const double* comp[9];
+                    for (int q = 0; q < nc; q++) comp[q] = dia_comp(h->full ? q : qmap3[q]);
+                    for (uint32_t w = 0; w < nt; w++) {
+                        const uint32_t r0 = 32 * w, r1 = std::min(n, r0 + 32);
+                        for (uint32_t d : diag_order) {
                             bool any = false;
-                            for (int q = 0; q < 9; q++) {
-                                const double* cp = dia_comp(q);
-                                if (cp) { v9[q] = cp[(size_t)d * n + i]; any |= v9[q] != 0.0; }
+                            for (uint32_t r = r0; r < r1 && !any; r++) {
+                                const int64_t col = (int64_t)r + doff[d];
+                                if (col < 0 || col >= (int64_t)n) continue;
+                                for (int q = 0; q < nc && !any; q++) any = comp[q][(size_t)d * n + r] != 0.0;
                             }
-                            if (!any) continue;
-                            ca.push_back((uint32_t)col);
-                            cv.insert(cv.end(), v9, v9 + 9);
+                            if (any) td.push_back(d);
                         }
-                        cx[i + 1] = (uint32_t)ca.size();
+                        tp[w + 1] = (uint32_t)td.size();
                     }
+                    h->dia.tile_ptr = dupload(tp.data(), tp.size());
+                    h->dia.tile_diag = dupload(td.data(), std::max<size_t>(td.size(), 1));
+                }
+                // the same matrix as SELL-32 for the fused kernels: rows take their entries in the
+                // order the DIA gather sums them in
+                {
+                    std::vector<uint32_t> cx, ca;
+                    std::vector<double> cv;
+                    dia_rows(n, s0.ndiag, doff, diag_order, dia_comp, cx, ca, cv);
                     build_sell(h, cx, ca, cv.data());
                     h->dexch = ASD_EXCH_CSR;
                 }

@@ -110,18 +110,24 @@ __constant__ double FRK5C[6] = {37.0 / 378.0, 0.0, 250.0 / 621.0, 125.0 / 594.0,
 __constant__ double FRK4C[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
 
 // Register caps of the FP32 kernels: 6 blocks of 256 per SM (40 registers) for the SELL and
-// the field-only kernels, 5 (48) for the DIA and the pattern kernels; the FP64 kernels keep the
-// default cap.  The pattern kernels have no staging state and gather six neighbours at once: at 40
-// registers their last stages spill and 96.2 µs per step became 91.6 at 48 (sc 128³, 300 K);
-// at 64 (4 blocks) the large lattices lose (24 replicas 120 → 152 µs per step).
+// the field-only kernels, 5 (48) for the DIA and the large pattern kernels, 4 (64) for the other
+// pattern kernels; the FP64 kernels keep the default cap.  The pattern kernels have no staging
+// state and hold six neighbours' loads in flight.  At 40 registers their last stages spill (sc
+// 128³ at 300 K: 93.6 µs per step, 90.9 at 48, 93.5 at 64; 24 replicas 119.6, 119.9, 129.6); lattices
+// of up to two waves of 4 blocks gain more from the loads in flight than they lose in warps (the
+// film 256×256×4 133.3 at 48, 127.1 at 64; sc 16³ 7.3, 7.2), and so do the full tensors (BCT-2 64³
+// 51.4 and 48.4, 37×29×23 15.7 and 14.8).
 // At 40 the diagonal-tensor SELL kernels spill 76 bytes a thread (the others none), and still
 // run faster than at 48: the extra warps hide more of the gather's latency than the spills add
 // (96 replicas 564 → 534 µs per step, the north star unchanged, A/B on one box).
 template <typename R, int EX, bool FULL, int K>
 struct MinBlocks {
     static constexpr int value =
-        sizeof(R) != 4 ? 1 : (EX == ASD_EXCH_DIA || EX == EXCH_PATTERN) ? 5 : 6;
+        sizeof(R) != 4 ? 1 : EX == EXCH_PATTERN_64 ? 4 : (EX == ASD_EXCH_DIA || EX == EXCH_PATTERN) ? 5 : 6;
 };
+constexpr uint32_t PATTERN_SMALL = 2 * 148 * 4 * 256;  // spins of two waves of 4 blocks of 256 per SM
+template <int EX>
+constexpr bool is_pattern = EX == EXCH_PATTERN || EX == EXCH_PATTERN_64;
 
 // K: the stage kind at compile time (1 Heun predictor, 2 Heun corrector, 3 RK stage before the
 // last, 4 last RK stage); a.kind still carries the RK stage index.
@@ -217,7 +223,7 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
     // 24 sc replicas (2.7 M spins) 155.0 → 121.6, sc 128×128×64 with dipole 175.9 → 163.0, BCT-2
     // 64³ 55.4 → 49.2, sc 16³ 8.9 → 7.7.
     uint32_t pid = 0;
-    if constexpr (EX == EXCH_PATTERN) {
+    if constexpr (is_pattern<EX>) {
         const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
         if (row < c.n) pid = __ldg(pat.row + row);
         if constexpr (FULL) load_table<R>(table_of<R>(sell), table_stride<FULL>() * sell.ntypes, tab);
@@ -302,11 +308,11 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
     R h[3] = {R(0), R(0), R(0)};
     // stage spin at this site; the pattern kernels load it with the gather's first loads
     R sv[3];
-    if constexpr (EX == EXCH_PATTERN)
+    if constexpr (is_pattern<EX>)
         for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
     if constexpr (EX == ASD_EXCH_CSR) gather_sell<R, FULL>(sell, i, a.src, tab, h, staged, wbase, sspin, staged16);
     if constexpr (EX == ASD_EXCH_DIA) gather_dia<R, FULL>(dia, c.n, i, a.src, tab, h);
-    if constexpr (EX == EXCH_PATTERN) gather_pattern<R, FULL>(pat, pid, i, a.src, tab, h);
+    if constexpr (is_pattern<EX>) gather_pattern<R, FULL>(pat, pid, i, a.src, tab, h);
     if (c.q4_ptr) {
         R h4[3];
         four_spin<R>(c, i, [&](uint32_t j, R v[3]) { v[0] = a.src.p[0][j]; v[1] = a.src.p[1][j]; v[2] = a.src.p[2][j]; }, h4);
@@ -330,7 +336,7 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
     h[1] += lrn[1] + dynr[DYN_APPLIED + 1];
     h[2] += lrn[2] + dynr[DYN_APPLIED + 2];
 
-    if constexpr (EX != EXCH_PATTERN)
+    if constexpr (!is_pattern<EX>)
         for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
     const int kind = a.kind;
     if constexpr (K >= 3) {
@@ -497,7 +503,7 @@ cudaError_t launch_stage_k(asd_handle* hd, const StageArgs<R>& a) {
             smem = ((smem + 15) & ~(size_t)15) + 4 * (size_t)hd->sell.stage_words;
         if (hd->sell.stage == 2) smem += 3 * sizeof(R) * (size_t)hd->sell.spin_slots;
     }
-    if (EX == EXCH_PATTERN && FULL) smem = sizeof(R) * table_stride<FULL>() * hd->sell.ntypes;
+    if (is_pattern<EX> && FULL) smem = sizeof(R) * table_stride<FULL>() * hd->sell.ntypes;
     if (EX == ASD_EXCH_DIA && hd->dia.dtype) smem = sizeof(R) * table_stride<FULL>() *hd->dia.ntypes;
     {
         const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(stage_kernel<R, EX, FULL, COMP, K>), smem);
@@ -511,9 +517,9 @@ cudaError_t launch_stage_k(asd_handle* hd, const StageArgs<R>& a) {
     }
     hd->launches += 1;
     if (hd->timing) {
-        const bool typed = (EX == ASD_EXCH_CSR && hd->sell.typed) || EX == EXCH_PATTERN || (EX == ASD_EXCH_DIA && hd->dia.dtype);
+        const bool typed = (EX == ASD_EXCH_CSR && hd->sell.typed) || is_pattern<EX> || (EX == ASD_EXCH_DIA && hd->dia.dtype);
         const std::string name = std::string("stage_kernel<") + (sizeof(R) == 4 ? "float" : "double") + "," +
-                                 (EX == ASD_EXCH_CSR ? "SELL32" : EX == EXCH_PATTERN ? "pattern" : EX == ASD_EXCH_DIA ? "DIA" : "NONE") +
+                                 (EX == ASD_EXCH_CSR ? "SELL32" : is_pattern<EX> ? "pattern" : EX == ASD_EXCH_DIA ? "DIA" : "NONE") +
                                  (typed ? "-typed" : "") + (FULL ? ",full" : ",diag") + (COMP ? ",comp" : "") +
                                  (K == 1 ? ",predictor>" : K == 2 ? ",corrector>" : K == 3 ? ",rk-stage>" : ",rk-last>");
         timer_end(hd, name, stage_bytes<R>(hd, a, COMP));
@@ -532,7 +538,10 @@ cudaError_t launch_stage_t(asd_handle* hd, const StageArgs<R>& a) {
 template <typename R, bool COMP>
 cudaError_t launch_stage(asd_handle* hd, const StageArgs<R>& a) {
     if (hd->dexch == ASD_EXCH_CSR && hd->sell.stage == STAGE_PATTERN) {
-        return hd->full ? launch_stage_t<R, EXCH_PATTERN, true, COMP>(hd, a) : launch_stage_t<R, EXCH_PATTERN, false, COMP>(hd, a);
+        if (hd->full) return launch_stage_t<R, EXCH_PATTERN_64, true, COMP>(hd, a);
+        if constexpr (sizeof(R) == 4)
+            if (hd->n > PATTERN_SMALL) return launch_stage_t<R, EXCH_PATTERN, false, COMP>(hd, a);
+        return launch_stage_t<R, EXCH_PATTERN_64, false, COMP>(hd, a);
     } else if (hd->dexch == ASD_EXCH_CSR) {
         return hd->full ? launch_stage_t<R, ASD_EXCH_CSR, true, COMP>(hd, a) : launch_stage_t<R, ASD_EXCH_CSR, false, COMP>(hd, a);
     } else if (hd->dexch == ASD_EXCH_DIA) {

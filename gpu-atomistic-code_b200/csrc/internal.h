@@ -50,16 +50,19 @@ struct SellDev {
 };
 // Row patterns of a typed matrix: the distinct sequences of (column - row, tensor id) over its
 // rows (a regular lattice has one per sublattice and boundary situation).  A row then costs its
-// 2-byte pattern number; the sequences, padded to W entries with (0, zero tensor), are read
-// through L1 by every row that follows them.  Entries keep the SELL order.
+// 2-byte pattern number; the sequences, padded to an even number W of entries with (0, zero
+// tensor), are read through L1, two entries per load, by every row that follows them.  Entries
+// keep the SELL order.
 struct PatDev {
     uint32_t W = 0;                  // entries per pattern (0: no patterns)
     uint32_t npat = 0;
     uint16_t* row = nullptr;         // pattern of each row
-    int2* ent = nullptr;             // [npat][W]: (column - row, tensor id)
+    int32_t* ent = nullptr;          // [npat][W]: (column - row) << 8 | tensor id
 };
+constexpr int32_t PAT_DELTA = 1 << 23;  // |column - row| is below this
 constexpr uint32_t STAGE_PATTERN = 3;   // SellDev::stage: the stage kernels gather by row patterns
-constexpr int EXCH_PATTERN = 4;         // the stage kernel's layout parameter in that mode
+// the stage kernel's layout parameter in that mode: at 48 registers, and at 64 (see MinBlocks)
+constexpr int EXCH_PATTERN = 4, EXCH_PATTERN_64 = 5;
 constexpr uint32_t MAG_CHUNK = 2048;  // spins per block of the magnetisation reduction
 constexpr uint32_t SPIN_PAD = 8;     // zeroed elements after every gather-source spin array
 

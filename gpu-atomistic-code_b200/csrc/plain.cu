@@ -3,6 +3,9 @@
 // the structure of the reference CUDA Heun (src/cuda.cu:43-258) and RK
 // (src/cudaRK4.cu:38-233, src/cudaRK5.cu) pipelines, written anew.
 //
+// A typed exchange matrix (few distinct tensors) runs each stage as one launch instead, in the same
+// arithmetic order (bct2 24³ cells, 300 K: PLAIN_A).
+//
 // This file is compiled with --fmad=false: every expression is evaluated
 // in the written order with correctly rounded operations, so the results
 // reproduce, bit for bit, an FP64 scalar CPU evaluation in the same order.
@@ -89,17 +92,17 @@ struct PlainSpin {
 
 // Total field of one spin (src/cuint.cu:66-137 order): CH + site + thermal + applied + anisotropy.
 __device__ __forceinline__ void plain_total_field(const StepConst& c, const PlainSpin& ps, uint32_t i,
-                                                  const double* ch, const double* rnd, const double s[3],
+                                                  const double ch[3], const double xi[3], const double s[3],
                                                   double h[3], double lrn[3]) {
     const uint32_t r = replica_of(c, i);
     const double TP = c.rep_sqrtT[r] * ps.sigma[i];
-    lrn[0] = rnd[3 * i] * TP;
-    lrn[1] = rnd[3 * i + 1] * TP;
-    lrn[2] = rnd[3 * i + 2] * TP;
+    lrn[0] = xi[0] * TP;
+    lrn[1] = xi[1] * TP;
+    lrn[2] = xi[2] * TP;
     const double* ap = c.dyn + DYN_APPLIED;
-    h[0] = ch[3 * i] + ps.hstg[3 * i] + lrn[0] + ap[0];
-    h[1] = ch[3 * i + 1] + ps.hstg[3 * i + 1] + lrn[1] + ap[1];
-    h[2] = ch[3 * i + 2] + ps.hstg[3 * i + 2] + lrn[2] + ap[2];
+    h[0] = ch[0] + ps.hstg[3 * i] + lrn[0] + ap[0];
+    h[1] = ch[1] + ps.hstg[3 * i + 1] + lrn[1] + ap[1];
+    h[2] = ch[2] + ps.hstg[3 * i + 2] + lrn[2] + ap[2];
     const double d[3] = {ps.k1udir[3 * i], ps.k1udir[3 * i + 1], ps.k1udir[3 * i + 2]};
     const double k1u = ps.k1u[i];
     const double sdn = s[0] * d[0] + s[1] * d[1] + s[2] * d[2];
@@ -143,7 +146,7 @@ __global__ void plain_heun1(StepConst c, PlainSpin ps, const double* __restrict_
     if (i >= c.n) return;
     const double s[3] = {sp[3 * i], sp[3 * i + 1], sp[3 * i + 2]};
     double h[3], lrn[3], f[3], e[3];
-    plain_total_field(c, ps, i, ch, rnd, s, h, lrn);
+    plain_total_field(c, ps, i, ch + 3 * (size_t)i, rnd + 3 * (size_t)i, s, h, lrn);
     plain_torque(1.0, ps.llgpf[i], ps.lambda[i], s, h, f);
     for (int j = 0; j < 3; j++) { fn[3 * i + j] = f[j]; e[j] = s[j] + f[j] * c.rdt; }
     plain_normalise(e);
@@ -158,7 +161,7 @@ __global__ void plain_heun2(StepConst c, PlainSpin ps, const double* __restrict_
     if (i >= c.n) return;
     const double e[3] = {es[3 * i], es[3 * i + 1], es[3 * i + 2]};
     double h[3], lrn[3], f[3], p[3];
-    plain_total_field(c, ps, i, ch, rnd, e, h, lrn);
+    plain_total_field(c, ps, i, ch + 3 * (size_t)i, rnd + 3 * (size_t)i, e, h, lrn);
     plain_torque(1.0, ps.llgpf[i], ps.lambda[i], e, h, f);
     for (int j = 0; j < 3; j++) p[j] = sp[3 * i + j] + (0.5 * (fn[3 * i + j] + f[j]) * c.rdt);
     plain_normalise(p);
@@ -182,20 +185,18 @@ __constant__ double RK5C[6] = {37.0 / 378.0, 0.0, 250.0 / 621.0, 125.0 / 594.0, 
 
 // One RK stage: k_st = rdt f(stage spin, H), next stage spin (src/cuintRK4.cu:62-434,
 // src/cuintRK5.cu:79-628 semantics; quirks selected by flags).
-__global__ void plain_rk_stage(StepConst c, PlainSpin ps, int nst, int st, const double* __restrict__ ch,
-                               const double* __restrict__ sp, double* __restrict__ es,
-                               const double* __restrict__ rnd, RkBufs kb) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;
+__device__ __forceinline__ void rk_stage_spin(const StepConst& c, const PlainSpin& ps, int nst, int st, uint32_t i,
+                                              const double ch[3], const double xi[3], const double* __restrict__ sp,
+                                              const double* src, double* dst, const RkBufs& kb) {
     const bool dbl = (c.flags & ASD_FLAG_RK_DOUBLE_RDT) != 0;
     const bool mixed = (c.flags & ASD_FLAG_RK_STAGE_SPIN_MIXED) != 0;
     const double S[3] = {sp[3 * i], sp[3 * i + 1], sp[3 * i + 2]};
     double sv[3];
     if (st == 0) { sv[0] = S[0]; sv[1] = S[1]; sv[2] = S[2]; }
-    else if (mixed) { sv[0] = es[3 * i]; sv[1] = S[1]; sv[2] = es[3 * i + 2]; }
-    else { sv[0] = es[3 * i]; sv[1] = es[3 * i + 1]; sv[2] = es[3 * i + 2]; }
+    else if (mixed) { sv[0] = src[3 * i]; sv[1] = S[1]; sv[2] = src[3 * i + 2]; }
+    else { sv[0] = src[3 * i]; sv[1] = src[3 * i + 1]; sv[2] = src[3 * i + 2]; }
     double h[3], lrn[3], k[3];
-    plain_total_field(c, ps, i, ch, rnd, sv, h, lrn);
+    plain_total_field(c, ps, i, ch, xi, sv, h, lrn);
     plain_torque(c.rdt, ps.llgpf[i], ps.lambda[i], sv, h, k);
     for (int j = 0; j < 3; j++) kb.k[st][3 * i + j] = k[j];
     if (st == nst - 1) return;
@@ -221,7 +222,130 @@ __global__ void plain_rk_stage(StepConst c, PlainSpin ps, int nst, int st, const
         e[j] = S[j] + inc;
     }
     plain_normalise(e);
-    es[3 * i] = e[0]; es[3 * i + 1] = e[1]; es[3 * i + 2] = e[2];
+    dst[3 * i] = e[0]; dst[3 * i + 1] = e[1]; dst[3 * i + 2] = e[2];
+}
+
+__global__ void plain_rk_stage(StepConst c, PlainSpin ps, int nst, int st, const double* __restrict__ ch,
+                               const double* __restrict__ sp, double* es, const double* __restrict__ rnd, RkBufs kb) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n) return;
+    rk_stage_spin(c, ps, nst, st, i, ch + 3 * (size_t)i, rnd + 3 * (size_t)i, sp, es, es, kb);
+}
+
+// ---- the exchange of a typed matrix (SellDev / PatDev), in the stage kernels themselves ----
+// sum_j J_ij S_j over the row's entries in their order, the products and sums of plain_spmv_csr /
+// plain_spmv_dia on the same values (exact zeros of a DIA matrix left out): the values come from
+// the table of distinct tensors, and the entries by row pattern (or, without patterns, as SELL
+// words read along the rows of a warp).  The CSR form above reads 76 bytes per full-tensor entry with
+// one row per thread, its warp's rows 2 KB apart.
+struct PlainTyped {
+    const uint32_t* xadj;      // row lengths
+    SellDev sell;
+    PatDev pat;
+};
+
+template <bool FULL, bool PAT>
+__device__ __forceinline__ void typed_row(const PlainTyped& m, const double* tab, uint32_t i,
+                                          const double* __restrict__ s, double dot[3]) {
+    dot[0] = dot[1] = dot[2] = 0.0;
+    const uint32_t len = m.xadj[i + 1] - m.xadj[i];
+    const uint32_t* w = nullptr;
+    const int32_t* e = nullptr;
+    if (PAT) e = m.pat.ent + (size_t)m.pat.row[i] * m.pat.W;
+    else w = m.sell.typed + m.sell.slice_ptr[i >> 5] + (i & 31u);
+    const uint32_t mask = PAT ? 0u : (1u << m.sell.colbits) - 1u;
+#pragma unroll 4
+    for (uint32_t k = 0; k < len; k++) {
+        uint32_t j, t;
+        if (PAT) {
+            const int32_t v = __ldg(e + k);
+            j = i + (uint32_t)(v >> 8);
+            t = (uint32_t)v & 255u;
+        } else {
+            const uint32_t v = __ldg(w + 32 * k);
+            j = v & mask;
+            t = v >> m.sell.colbits;
+        }
+        const double x = __ldg(s + 3 * (size_t)j), y = __ldg(s + 3 * (size_t)j + 1), z = __ldg(s + 3 * (size_t)j + 2);
+        const double* T = tab + (FULL ? 12u : 4u) * t;
+        if (!FULL) {
+            dot[0] += T[0] * x;
+            dot[1] += T[1] * y;
+            dot[2] += T[2] * z;
+        } else {
+#pragma unroll
+            for (int co = 0; co < 3; co++) {
+                dot[co] += T[3 * co] * x;
+                dot[co] += T[3 * co + 1] * y;
+                dot[co] += T[3 * co + 2] * z;
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void load_tab(const SellDev& m, uint32_t stride, double* tab) {
+    for (uint32_t q = threadIdx.x; q < stride * m.ntypes; q += blockDim.x) tab[q] = m.tab_d[q];
+    __syncthreads();
+}
+
+template <bool FULL, bool PAT>
+__global__ void plain_spmv_typed(uint32_t n, const PlainTyped m, const double* __restrict__ s,
+                                 const double* __restrict__ hd, double* __restrict__ ch) {
+    extern __shared__ double tab[];
+    load_tab(m.sell, FULL ? 12 : 4, tab);
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double dot[3];
+    typed_row<FULL, PAT>(m, tab, i, s, dot);
+    for (int a = 0; a < 3; a++) ch[3 * (size_t)i + a] = hd[3 * (size_t)i + a] + dot[a];
+}
+
+// One stage in one launch: exchange, the step's noise (drawn and stored by the first stage; a
+// replica at T = 0 draws none, its thermal field being zero), total field, torque and update.  KIND 1, 2: Heun
+// predictor, corrector; 3: RK stage `st`, whose spins go to a second buffer (`dst`), since other
+// blocks still gather from `src`.
+template <bool FULL, bool PAT, int KIND>
+__global__ void __launch_bounds__(128) plain_stage_typed(const StepConst c, const PlainSpin ps, const PlainTyped m,
+                                                         uint64_t step, int nst, int st, const double* __restrict__ hd,
+                                                         double* sp, const double* src, double* dst, double* rnd,
+                                                         double* fn, double* det, const RkBufs kb) {
+    extern __shared__ double tab[];
+    load_tab(m.sell, FULL ? 12 : 4, tab);
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n) return;
+    double ch[3], xi[3] = {0.0, 0.0, 0.0};
+    typed_row<FULL, PAT>(m, tab, i, KIND == 1 || (KIND == 3 && st == 0) ? sp : src, ch);
+    for (int a = 0; a < 3; a++) ch[a] = hd[3 * (size_t)i + a] + ch[a];
+    const uint32_t r = replica_of(c, i);
+    if (c.rep_sqrtT[r] != 0.0) {
+        if (KIND == 1 || (KIND == 3 && st == 0)) {
+            thermal_normals(c.seed, c.rep_stream[r], i - c.rep_off[r], step, xi);
+            for (int a = 0; a < 3; a++) rnd[3 * (size_t)i + a] = xi[a];
+        } else {
+            for (int a = 0; a < 3; a++) xi[a] = rnd[3 * (size_t)i + a];
+        }
+    }
+    if constexpr (KIND == 3) {
+        rk_stage_spin(c, ps, nst, st, i, ch, xi, sp, src, dst, kb);
+    } else {
+        const double* at = KIND == 1 ? sp : src;
+        const double s[3] = {at[3 * i], at[3 * i + 1], at[3 * i + 2]};
+        double h[3], lrn[3], f[3], e[3];
+        plain_total_field(c, ps, i, ch, xi, s, h, lrn);
+        plain_torque(1.0, ps.llgpf[i], ps.lambda[i], s, h, f);
+        if constexpr (KIND == 1) {
+            for (int j = 0; j < 3; j++) { fn[3 * i + j] = f[j]; e[j] = s[j] + f[j] * c.rdt; }
+            plain_normalise(e);
+            for (int j = 0; j < 3; j++) dst[3 * i + j] = e[j];
+        } else {
+            for (int j = 0; j < 3; j++) e[j] = sp[3 * i + j] + (0.5 * (fn[3 * i + j] + f[j]) * c.rdt);
+            plain_normalise(e);
+            for (int j = 0; j < 3; j++) {
+                sp[3 * i + j] = e[j];
+                det[3 * i + j] = h[j] - lrn[j];
+            }
+        }
+    }
 }
 
 // Final combination + renormalisation (CdetSnp1, src/cuintRK4.cu:436-456, src/cuintRK5.cu:630-649).
@@ -343,6 +467,16 @@ static cudaError_t plain_field_exch(asd_handle* h, const double* s, double* ch) 
     cudaStream_t st = h->stream;
     const int zz = (h->p.flags & ASD_FLAG_GPU_DZZ_FROM_DYY) ? 1 : 0;
     if (h->lr.mode == ASD_LR_FFT) return launch_lr_eval_plain(h, s, ch, false);
+    if (h->sell.typed) {
+        const PlainTyped m{h->pex.xadj, h->sell, h->pat};
+        const size_t sm = sizeof(double) * (h->full ? 12 : 4) * h->sell.ntypes;
+        if (h->full && h->pat.W) plain_spmv_typed<true, true><<<nb(h->n, B), B, sm, st>>>(h->n, m, s, h->p_hdemag, ch);
+        else if (h->full) plain_spmv_typed<true, false><<<nb(h->n, B), B, sm, st>>>(h->n, m, s, h->p_hdemag, ch);
+        else if (h->pat.W) plain_spmv_typed<false, true><<<nb(h->n, B), B, sm, st>>>(h->n, m, s, h->p_hdemag, ch);
+        else plain_spmv_typed<false, false><<<nb(h->n, B), B, sm, st>>>(h->n, m, s, h->p_hdemag, ch);
+        h->launches += 1;
+        return cudaGetLastError();
+    }
     if (h->exch == ASD_EXCH_CSR) {
         if (h->full) plain_spmv_csr<true><<<nb(h->n, B), B, 0, st>>>(h->n, h->pex.xadj, h->pex.adjncy, h->pex, s, h->p_hdemag, ch, zz);
         else plain_spmv_csr<false><<<nb(h->n, B), B, 0, st>>>(h->n, h->pex.xadj, h->pex.adjncy, h->pex, s, h->p_hdemag, ch, zz);
@@ -352,6 +486,27 @@ static cudaError_t plain_field_exch(asd_handle* h, const double* s, double* ch) 
     } else {
         cudaMemcpyAsync(ch, h->p_hdemag, 3 * (size_t)h->n * sizeof(double), cudaMemcpyDeviceToDevice, st);
         return cudaGetLastError();
+    }
+    h->launches += 1;
+    return cudaGetLastError();
+}
+
+// One stage of a typed matrix (KIND as in plain_stage_typed).
+template <int KIND>
+static cudaError_t launch_stage_typed(asd_handle* h, uint64_t t, int nst, int st, const double* src, double* dst,
+                                      const RkBufs& kb) {
+    const PlainSpin ps{h->p_sigma, h->p_llgpf, h->p_lambda, h->p_k1u, h->p_k1udir, h->p_hstg};
+    const PlainTyped m{h->pex.xadj, h->sell, h->pat};
+    const size_t sm = sizeof(double) * (h->full ? 12 : 4) * h->sell.ntypes;
+    const unsigned g = nb(h->n, 128);
+    auto run = [&](auto kern) {
+        kern<<<g, 128, sm, h->stream>>>(h->sc, ps, m, t, nst, st, h->p_hdemag, h->p_s, src, dst, h->p_rand, h->p_fn,
+                                        h->p_det, kb);
+    };
+    if (h->full) {
+        if (h->pat.W) run(plain_stage_typed<true, true, KIND>); else run(plain_stage_typed<true, false, KIND>);
+    } else {
+        if (h->pat.W) run(plain_stage_typed<false, true, KIND>); else run(plain_stage_typed<false, false, KIND>);
     }
     h->launches += 1;
     return cudaGetLastError();
@@ -371,15 +526,35 @@ cudaError_t launch_plain_step(asd_handle* h, uint64_t t) {
         const double f = h->pulse_amp * exp(-0.5 * x * x);
         if ((e = launch_plain_ramp(h, h->stag_rv * f)) != cudaSuccess) return e;
     }
+    // A typed matrix runs each stage as one launch (Heun 2 instead of 5, no field array in between);
+    // the four-spin term and the stale-corrector flag need the field as a pass of its own.
+    const bool stale_flag = (h->p.flags & ASD_FLAG_GPU_CSR_DIP_STALE) && h->lr.mode == ASD_LR_DIPOLE &&
+                            h->exch == ASD_EXCH_CSR && !h->full;
+    const bool typed = h->sell.typed && h->lr.mode != ASD_LR_FFT && !h->sc.q4_ptr;
+    if (typed && !(h->p.integrator == ASD_HEUN && stale_flag)) {
+        RkBufs kb;
+        for (int q = 0; q < 6; q++) kb.k[q] = h->p_k[q];
+        if (dip_refresh && (e = launch_lr_eval_plain(h, h->p_s, h->p_hdemag, true)) != cudaSuccess) return e;
+        if (h->p.integrator == ASD_HEUN) {
+            if ((e = launch_stage_typed<1>(h, t, 0, 0, h->p_es, h->p_es, kb)) != cudaSuccess) return e;
+            return launch_stage_typed<2>(h, t, 0, 0, h->p_es, h->p_es, kb);
+        }
+        const int nst = h->p.integrator == ASD_RK4 ? 4 : 6;
+        double* pp[2] = {h->p_es, h->p_fn};           // stage spins alternate between two buffers
+        for (int q = 0; q < nst; q++)
+            if ((e = launch_stage_typed<3>(h, t, nst, q, q ? pp[(q - 1) & 1] : h->p_s, pp[q & 1], kb)) != cudaSuccess)
+                return e;
+        plain_rk_final<<<nb(h->n, B), B, 0, st>>>(h->n, nst, h->p_s, kb);
+        h->launches += 1;
+        return cudaGetLastError();
+    }
     if (h->p.integrator == ASD_HEUN) {
         if (dip_refresh && (e = launch_lr_eval_plain(h, h->p_s, h->p_hdemag, true)) != cudaSuccess) return e;
         if ((e = plain_field(h, h->p_s, h->p_ch)) != cudaSuccess) return e;
         plain_noise_k<<<nb(h->n, B), B, 0, st>>>(h->sc, t, h->p_rand);
         plain_heun1<<<nb(h->n, B), B, 0, st>>>(h->sc, ps, h->p_ch, h->p_s, h->p_es, h->p_rand, h->p_fn);
         h->launches += 2;
-        const bool stale = (h->p.flags & ASD_FLAG_GPU_CSR_DIP_STALE) && h->lr.mode == ASD_LR_DIPOLE &&
-                           h->exch == ASD_EXCH_CSR && !h->full;
-        if (!stale && (e = plain_field(h, h->p_es, h->p_ch)) != cudaSuccess) return e;
+        if (!stale_flag && (e = plain_field(h, h->p_es, h->p_ch)) != cudaSuccess) return e;
         plain_heun2<<<nb(h->n, B), B, 0, st>>>(h->sc, ps, h->p_ch, h->p_s, h->p_es, h->p_rand, h->p_fn, h->p_det);
         h->launches += 1;
         return cudaGetLastError();
