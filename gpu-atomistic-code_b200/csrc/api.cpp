@@ -200,7 +200,7 @@ void build_patterns(asd_handle* h, const std::vector<uint32_t>& xadj, const std:
 }
 
 // CSR (all replicas concatenated) -> SELL-32 device layout.
-void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vector<uint32_t>& adj0,
+void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vector<uint32_t>& adj,
                 const double* val9) {
     const uint32_t n = h->n;
     const bool full = h->full != 0;
@@ -226,9 +226,9 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
         const int nc = full ? 9 : 3;
         const int qmap[9] = {0, 4, 8, 0, 0, 0, 0, 0, 0};
         TensorTable tt(nc);
-        std::vector<uint32_t> id(adj0.size());
+        std::vector<uint32_t> id(adj.size());
         bool ok = true;
-        for (size_t k = 0; k < adj0.size() && ok; k++) {
+        for (size_t k = 0; k < adj.size() && ok; k++) {
             std::array<double, 9> key{};
             for (int q = 0; q < nc; q++) key[q] = value((uint32_t)k, full ? q : qmap[q]);
             const int64_t t = tt.id(key);
@@ -236,23 +236,6 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
         }
         const uint32_t tb = tt.bits();
         if (ok && (uint64_t)n <= (1ull << (32 - tb))) {
-            // full tensors: a row's entries by tensor (RowSum), in the caller's order within one; DIA
-            // input comes in its diagonals' order by tensor already (diag_order)
-            std::vector<uint32_t> col_by;
-            if (full && h->exch == ASD_EXCH_CSR && h->p.precision != ASD_FP64_PLAIN) {
-                col_by = adj0;
-                std::vector<std::pair<uint32_t, uint32_t>> rowv;
-                for (uint32_t r = 0; r < n; r++) {
-                    const uint32_t e0 = xadj[r], e1 = xadj[r + 1];
-                    if (std::is_sorted(id.begin() + e0, id.begin() + e1)) continue;
-                    rowv.clear();
-                    for (uint32_t k = e0; k < e1; k++) rowv.emplace_back(id[k], adj0[k]);
-                    std::stable_sort(rowv.begin(), rowv.end(),
-                                     [](const auto& a, const auto& b) { return a.first < b.first; });
-                    for (uint32_t k = e0; k < e1; k++) { id[k] = rowv[k - e0].first; col_by[k] = rowv[k - e0].second; }
-                }
-            }
-            const std::vector<uint32_t>& adj = col_by.empty() ? adj0 : col_by;
             std::vector<uint32_t> w(E);
             for (uint32_t s = 0; s < ns; s++) {
                 const uint32_t wd = (sp[s + 1] - sp[s]) / 32;
@@ -292,7 +275,7 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
                     float v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
                     if (r < n && k < xadj[r + 1] - xadj[r]) {
                         const uint32_t kk = xadj[r] + k;
-                        col = (int)adj0[kk];
+                        col = (int)adj[kk];
                         for (int q = 0; q < 9; q++) v[q] = (float)value(kk, q);
                     }
                     int ci;
@@ -322,7 +305,7 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
                     col[e] = r < n ? (int)r : 0;
                     if (r < n && k < xadj[r + 1] - xadj[r]) {
                         const uint32_t kk = xadj[r] + k;
-                        col[e] = (int)adj0[kk];
+                        col[e] = (int)adj[kk];
                         for (int q = 0; q < nc; q++) v[(size_t)q * E + e] = value(kk, full ? q : qmap3[q]);
                     }
                 }
@@ -332,15 +315,14 @@ void build_sell(asd_handle* h, const std::vector<uint32_t>& xadj, const std::vec
     }
 }
 
-// The rows of a DIA matrix as CSR, entries in the diagonals' `order`, exact zeros left out.
+// The rows of a DIA matrix as CSR, entries in ascending diagonal order, exact zeros left out.
 template <typename Comp>
-void dia_rows(uint32_t n, uint32_t ndiag, const std::vector<int32_t>& doff, const std::vector<uint32_t>& order,
-              Comp comp, std::vector<uint32_t>& cx, std::vector<uint32_t>& ca, std::vector<double>& cv) {
+void dia_rows(uint32_t n, uint32_t ndiag, const std::vector<int32_t>& doff, Comp comp, std::vector<uint32_t>& cx, std::vector<uint32_t>& ca, std::vector<double>& cv) {
     cx.assign((size_t)n + 1, 0);
     const double* cp[9];
     for (int q = 0; q < 9; q++) cp[q] = ndiag ? comp(q) : nullptr;
     for (uint32_t i = 0; i < n; i++) {
-        for (uint32_t d : order) {
+        for (uint32_t d = 0; d < ndiag; d++) {
             const int64_t col = (int64_t)i + doff[d];
             if (col < 0 || col >= (int64_t)n) continue;
             double v9[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
@@ -1100,9 +1082,7 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
             } else if (h->exch == ASD_EXCH_DIA) {
                 std::vector<uint32_t> cx, ca;
                 std::vector<double> cv;
-                std::vector<uint32_t> order(s0.ndiag);
-                for (uint32_t d = 0; d < s0.ndiag; d++) order[d] = d;
-                dia_rows(n, s0.ndiag, doff, order, dia_comp, cx, ca, cv);
+                dia_rows(n, s0.ndiag, doff, dia_comp, cx, ca, cv);
                 h->pex.xadj = dupload(cx.data(), cx.size());
                 build_sell(h, cx, ca, cv.data());
                 if (!h->sell.typed) {
@@ -1146,8 +1126,6 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
                 const int nc = h->full ? 9 : 3;
                 const int qmap3[3] = {0, 4, zz_yy ? 4 : 8};
                 bool typed = false;
-                std::vector<uint32_t> diag_order(s0.ndiag);   // the order the gathers take the diagonals in
-                for (uint32_t d = 0; d < s0.ndiag; d++) diag_order[d] = d;
                 if (!(p.flags & ASD_FLAG_STREAMED_EXCHANGE)) {
                     // typed DIA: one id byte per (diagonal, row) into the distinct tensors
                     TensorTable tt(nc);
@@ -1164,19 +1142,6 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
                     if (ok) {
                         h->dia.dtype = dupload(ids.data(), ids.size());
                         h->dia.ntypes = tt.size();
-                        if (h->full) {
-                            // full tensors: the diagonals by their smallest tensor id, so that the
-                            // entries of one tensor follow each other in the rows (RowSum)
-                            std::vector<uint32_t> key(s0.ndiag, 256);
-                            for (uint32_t d = 0; d < s0.ndiag; d++)
-                                for (uint32_t i = 0; i < n; i++) {
-                                    const int64_t col = (int64_t)i + doff[d];
-                                    const uint32_t t = ids[(size_t)d * n + i];
-                                    if (t && t < key[d] && col >= 0 && col < (int64_t)n) key[d] = t;
-                                }
-                            std::stable_sort(diag_order.begin(), diag_order.end(),
-                                             [&](uint32_t a, uint32_t b) { return key[a] < key[b]; });
-                        }
                         if (bytes == 4) { std::vector<float> tf = tt.table<float>(); h->dia.tab_f = dupload(tf.data(), tf.size()); }
                         else { std::vector<double> td = tt.table<double>(); h->dia.tab_d = dupload(td.data(), td.size()); }
                         typed = true;
@@ -1209,7 +1174,7 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
                     for (int q = 0; q < nc; q++) comp[q] = dia_comp(h->full ? q : qmap3[q]);
                     for (uint32_t w = 0; w < nt; w++) {
                         const uint32_t r0 = 32 * w, r1 = std::min(n, r0 + 32);
-                        for (uint32_t d : diag_order) {
+                        for (uint32_t d = 0; d < s0.ndiag; d++) {
                             bool any = false;
                             for (uint32_t r = r0; r < r1 && !any; r++) {
                                 const int64_t col = (int64_t)r + doff[d];
@@ -1223,12 +1188,12 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
                     h->dia.tile_ptr = dupload(tp.data(), tp.size());
                     h->dia.tile_diag = dupload(td.data(), std::max<size_t>(td.size(), 1));
                 }
-                // the same matrix as SELL-32 for the fused kernels: rows take their entries in the
-                // order the DIA gather sums them in
+                // the same matrix as SELL-32 for the fused kernels: rows take their entries in
+                // ascending diagonal order, the order the DIA gather sums them in
                 {
                     std::vector<uint32_t> cx, ca;
                     std::vector<double> cv;
-                    dia_rows(n, s0.ndiag, doff, diag_order, dia_comp, cx, ca, cv);
+                    dia_rows(n, s0.ndiag, doff, dia_comp, cx, ca, cv);
                     build_sell(h, cx, ca, cv.data());
                     h->dexch = ASD_EXCH_CSR;
                 }

@@ -110,24 +110,25 @@ __constant__ double FRK5C[6] = {37.0 / 378.0, 0.0, 250.0 / 621.0, 125.0 / 594.0,
 __constant__ double FRK4C[4] = {1.0 / 6.0, 1.0 / 3.0, 1.0 / 3.0, 1.0 / 6.0};
 
 // Register caps of the FP32 kernels: 6 blocks of 256 per SM (40 registers) for the SELL and
-// the field-only kernels, 5 (48) for the DIA and the large pattern kernels, 4 (64) for the other
+// the field-only kernels, 5 (48) for the DIA and some pattern kernels, 4 (64) for the other
 // pattern kernels; the FP64 kernels keep the default cap.  The pattern kernels have no staging
 // state and hold six neighbours' loads in flight.  At 40 registers their last stages spill (sc
-// 128³ at 300 K: 93.6 µs per step, 90.9 at 48, 93.5 at 64; 24 replicas 119.6, 119.9, 129.6); lattices
-// of up to two waves of 4 blocks gain more from the loads in flight than they lose in warps (the
-// film 256×256×4 133.3 at 48, 127.1 at 64; sc 16³ 7.3, 7.2), and so do the full tensors (BCT-2 64³
-// 51.4 and 48.4, 37×29×23 15.7 and 14.8).
+// 128³ at 300 K: 93.6 µs per step, 90.9 at 48, 93.5 at 64; 24 replicas 119.6, 119.9, 129.6; sc
+// 90×75×41 with dipole 70.6 at 48, 73.6 at 64).  64 where a row takes several batches of loads: up
+// to two waves of 4 blocks (the film 256×256×4, 18 neighbours: 133.3 at 48, 127.1 at 64) and full
+// tensors (BCT-2 64³ 48.9 and 48.7, 37×29×23 15.7 and 14.8); and up to one wave, where nothing is
+// lost (sc 16³ 7.3, 7.2).
 // At 40 the diagonal-tensor SELL kernels spill 76 bytes a thread (the others none), and still
 // run faster than at 48: the extra warps hide more of the gather's latency than the spills add
 // (96 replicas 564 → 534 µs per step, the north star unchanged, A/B on one box).
 template <typename R, int EX, bool FULL, int K>
 struct MinBlocks {
     static constexpr int value =
-        sizeof(R) != 4 ? 1 : EX == EXCH_PATTERN_64 ? 4 : (EX == ASD_EXCH_DIA || EX == EXCH_PATTERN) ? 5 : 6;
+        sizeof(R) != 4 ? 1 : EX == EXCH_PATTERN_64 || EX == EXCH_PATTERN_EARLY ? 4 : (EX == ASD_EXCH_DIA || EX == EXCH_PATTERN) ? 5 : 6;
 };
-constexpr uint32_t PATTERN_SMALL = 2 * 148 * 4 * 256;  // spins of two waves of 4 blocks of 256 per SM
+constexpr uint32_t PATTERN_WAVE = 148 * 4 * 256;       // spins of one wave of 4 blocks of 256 per SM
 template <int EX>
-constexpr bool is_pattern = EX == EXCH_PATTERN || EX == EXCH_PATTERN_64;
+constexpr bool is_pattern = EX == EXCH_PATTERN || EX == EXCH_PATTERN_64 || EX == EXCH_PATTERN_EARLY;
 
 // K: the stage kind at compile time (1 Heun predictor, 2 Heun corrector, 3 RK stage before the
 // last, 4 last RK stage); a.kind still carries the RK stage index.
@@ -222,10 +223,20 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
     // staged SELL shapes (step time in the graph, one B200): sc 128³ at 300 K 119.2 → 91.6 µs,
     // 24 sc replicas (2.7 M spins) 155.0 → 121.6, sc 128×128×64 with dipole 175.9 → 163.0, BCT-2
     // 64³ 55.4 → 49.2, sc 16³ 8.9 → 7.7.
+    // EARLY (FP32 lattices of at most one wave): the time of a stage is its chain of dependent loads,
+    // so the pattern's first words are read before the dependent-launch wait and their neighbours
+    // right after it, ahead of the thermal draw, and no L2 prefetch is issued (the state is in L2).
+    // µs per step: sc 16³ at 300 K 7.16 → 6.78, BCT-2 37×29×23 14.7 → 13.0; in FP64 (72 registers of
+    // neighbours held across the draw) it loses: 64×64×32 with dipole 45.7 → 47.6.
+    constexpr bool EARLY = EX == EXCH_PATTERN_EARLY;
+    const bool early = EARLY && pat.W >= PAT_BATCH;
+    PatBatch<R, PAT_BATCH> first;
     uint32_t pid = 0;
     if constexpr (is_pattern<EX>) {
         const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
         if (row < c.n) pid = __ldg(pat.row + row);
+        if constexpr (EARLY)
+            if (early && row < c.n) first.words(reinterpret_cast<const int2*>(pat.ent + (size_t)pid * pat.W));
         if constexpr (FULL) load_table<R>(table_of<R>(sell), table_stride<FULL>() * sell.ntypes, tab);
         else tab = const_cast<R*>(table_of<R>(sell));
     }
@@ -240,7 +251,7 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
                           &stage_bar);
             }
     }
-    if (threadIdx.x == 0 && a.npf) {
+    if (!EARLY && threadIdx.x == 0 && a.npf) {
         // the block's rows of every per-spin input: one bulk L2 prefetch each, so the loads
         // after the exchange gather find them in L2; sizes stop at the last row (whole
         // 16-byte units), so no prefetch reaches past an array
@@ -253,6 +264,12 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
     }
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;     // thread 0 of every block has i < n and always waits below
+    // stage spin at this site; the pattern kernels load it with the gather's first loads
+    R sv[3];
+    if constexpr (EARLY) {
+        for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
+        if (early) first.spins(i, a.src);
+    }
     const uint64_t t = *c.step_base + a.rel;
     const uint32_t at = atom_of(c, i);
     const MatConst& mc = c.mat[at];
@@ -306,13 +323,14 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
         stage_timeout = true;
     }
     R h[3] = {R(0), R(0), R(0)};
-    // stage spin at this site; the pattern kernels load it with the gather's first loads
-    R sv[3];
-    if constexpr (is_pattern<EX>)
+    if constexpr (is_pattern<EX> && !EARLY)
         for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
     if constexpr (EX == ASD_EXCH_CSR) gather_sell<R, FULL>(sell, i, a.src, tab, h, staged, wbase, sspin, staged16);
     if constexpr (EX == ASD_EXCH_DIA) gather_dia<R, FULL>(dia, c.n, i, a.src, tab, h);
-    if constexpr (is_pattern<EX>) gather_pattern<R, FULL>(pat, pid, i, a.src, tab, h);
+    if constexpr (is_pattern<EX>) {
+        if (early) first.template add<FULL>(tab, h);
+        gather_pattern<R, FULL>(pat, pid, i, a.src, tab, h, early ? PAT_BATCH : 0u);
+    }
     if (c.q4_ptr) {
         R h4[3];
         four_spin<R>(c, i, [&](uint32_t j, R v[3]) { v[0] = a.src.p[0][j]; v[1] = a.src.p[1][j]; v[2] = a.src.p[2][j]; }, h4);
@@ -538,10 +556,15 @@ cudaError_t launch_stage_t(asd_handle* hd, const StageArgs<R>& a) {
 template <typename R, bool COMP>
 cudaError_t launch_stage(asd_handle* hd, const StageArgs<R>& a) {
     if (hd->dexch == ASD_EXCH_CSR && hd->sell.stage == STAGE_PATTERN) {
-        if (hd->full) return launch_stage_t<R, EXCH_PATTERN_64, true, COMP>(hd, a);
-        if constexpr (sizeof(R) == 4)
-            if (hd->n > PATTERN_SMALL) return launch_stage_t<R, EXCH_PATTERN, false, COMP>(hd, a);
-        return launch_stage_t<R, EXCH_PATTERN_64, false, COMP>(hd, a);
+        if constexpr (sizeof(R) == 4) {
+            if (hd->n <= PATTERN_WAVE)
+                return hd->full ? launch_stage_t<R, EXCH_PATTERN_EARLY, true, COMP>(hd, a)
+                                : launch_stage_t<R, EXCH_PATTERN_EARLY, false, COMP>(hd, a);
+            if (!hd->full && (hd->n > 2 * PATTERN_WAVE || hd->pat.W <= PAT_BATCH))
+                return launch_stage_t<R, EXCH_PATTERN, false, COMP>(hd, a);
+        }
+        return hd->full ? launch_stage_t<R, EXCH_PATTERN_64, true, COMP>(hd, a)
+                        : launch_stage_t<R, EXCH_PATTERN_64, false, COMP>(hd, a);
     } else if (hd->dexch == ASD_EXCH_CSR) {
         return hd->full ? launch_stage_t<R, ASD_EXCH_CSR, true, COMP>(hd, a) : launch_stage_t<R, ASD_EXCH_CSR, false, COMP>(hd, a);
     } else if (hd->dexch == ASD_EXCH_DIA) {

@@ -10,7 +10,6 @@
 //    The table is staged in shared memory, component-major [c][ntypes].
 #pragma once
 #include "internal.h"
-#include <type_traits>
 
 namespace asd {
 
@@ -140,34 +139,6 @@ __device__ __forceinline__ void accumulate_typed(const R* tab, uint32_t t, R x, 
     }
 }
 
-// h += sum of J_t S over a row's entries, taken in order.  Full tensors: consecutive entries of one
-// tensor are summed first and multiplied once (a shell of a lattice shares its tensor: BCT-2 has
-// 26 neighbours and 7 products, 3 adds and a compare per neighbour in place of 9 multiply-adds
-// and three 16-byte table loads); the rows' entries are ordered by tensor for it.  Every layout forms
-// the same sums.
-template <typename R, bool FULL>
-struct RowSum {
-    uint32_t cur = 0;
-    R s[3] = {R(0), R(0), R(0)};
-    __device__ __forceinline__ void add(const R* tab, uint32_t t, R x, R y, R z, R h[3]) {
-        if constexpr (FULL) {
-            if (t != cur) {
-                finish(tab, h);
-                cur = t;
-                s[0] = R(0); s[1] = R(0); s[2] = R(0);
-            }
-            s[0] += x; s[1] += y; s[2] += z;
-        } else {
-            accumulate_typed<R, false>(tab, t, x, y, z, h);
-        }
-    }
-    __device__ __forceinline__ void finish(const R* tab, R h[3]) {
-        if constexpr (FULL) {
-            if (cur) accumulate_typed<R, true>(tab, cur, s[0], s[1], s[2], h);
-        }
-    }
-};
-
 // h += sum over the row's entries of J_e S_col(e), SELL-32 layout (one warp per slice).
 template <typename R, bool FULL>
 __device__ __forceinline__ void gather_sell(const SellDev& m, uint32_t i, const CVec3<R>& s, const R* tab, R h[3],
@@ -175,7 +146,6 @@ __device__ __forceinline__ void gather_sell(const SellDev& m, uint32_t i, const 
                                             const R* sspin = nullptr, const uint16_t* staged16 = nullptr) {
     const uint32_t sl = i >> 5, lane = i & 31u;
     const uint32_t p0 = __ldg(m.slice_ptr + sl), p1 = __ldg(m.slice_ptr + sl + 1);
-    RowSum<R, FULL> rs;
     if (m.typed && staged16 && sspin) {
         // 16-bit words: slot | id << lbits into the staged neighbour spins [3][spin_slots]
         const uint32_t mask = (1u << m.lbits) - 1u, cb = m.lbits, ns = m.spin_slots;
@@ -183,9 +153,8 @@ __device__ __forceinline__ void gather_sell(const SellDev& m, uint32_t i, const 
         for (uint32_t e = p0 - wbase + lane; e < p1 - wbase; e += 32) {
             const uint32_t w = staged16[e];
             const uint32_t j = w & mask, t = w >> cb;
-            rs.add(tab, t, sspin[j], sspin[ns + j], sspin[2 * ns + j], h);
+            accumulate_typed<R, FULL>(tab, t, sspin[j], sspin[ns + j], sspin[2 * ns + j], h);
         }
-        rs.finish(tab, h);
         return;
     }
     if (m.typed && staged && sspin) {
@@ -195,9 +164,8 @@ __device__ __forceinline__ void gather_sell(const SellDev& m, uint32_t i, const 
         for (uint32_t e = p0 - wbase + lane; e < p1 - wbase; e += 32) {
             const uint32_t w = staged[e];
             const uint32_t j = w & mask, t = w >> cb;
-            rs.add(tab, t, sspin[j], sspin[ns + j], sspin[2 * ns + j], h);
+            accumulate_typed<R, FULL>(tab, t, sspin[j], sspin[ns + j], sspin[2 * ns + j], h);
         }
-        rs.finish(tab, h);
         return;
     }
     if (m.typed && staged) {
@@ -208,9 +176,8 @@ __device__ __forceinline__ void gather_sell(const SellDev& m, uint32_t i, const 
             const uint32_t w = staged[e];
             const uint32_t j = w & mask, t = w >> cb;
             const R x = __ldg(s.p[0] + j), y = __ldg(s.p[1] + j), z = __ldg(s.p[2] + j);
-            rs.add(tab, t, x, y, z, h);
+            accumulate_typed<R, FULL>(tab, t, x, y, z, h);
         }
-        rs.finish(tab, h);
         return;
     }
     if (m.typed) {
@@ -220,9 +187,8 @@ __device__ __forceinline__ void gather_sell(const SellDev& m, uint32_t i, const 
             const uint32_t w = ldcs(m.typed + e);
             const uint32_t j = w & mask, t = w >> cb;
             const R x = __ldg(s.p[0] + j), y = __ldg(s.p[1] + j), z = __ldg(s.p[2] + j);
-            rs.add(tab, t, x, y, z, h);
+            accumulate_typed<R, FULL>(tab, t, x, y, z, h);
         }
-        rs.finish(tab, h);
         return;
     }
     if constexpr (sizeof(R) == 4) {
@@ -262,39 +228,56 @@ __device__ __forceinline__ void gather_sell(const SellDev& m, uint32_t i, const 
     }
 }
 
-constexpr uint32_t PAT_BATCH = 6;                      // (full tensors: 4 measured 3 % slower on BCT-2 64³)
+constexpr uint32_t PAT_BATCH = 6;
 
-// h += sum over the row's pattern of J_id S_{i + delta}; `tab` is the tensor table (global memory
-// for the diagonal form, whose few rows stay in L1; shared memory for full tensors).
-template <typename R, bool FULL>
-__device__ __forceinline__ void gather_pattern(const PatDev& m, uint32_t pid, uint32_t i, const CVec3<R>& s,
-                                               const R* tab, R h[3]) {
-    RowSum<R, FULL> rs;
-    // U entries' loads are issued before the first of them is used
-    constexpr uint32_t U = PAT_BATCH;
-    const int2* __restrict__ e = reinterpret_cast<const int2*>(m.ent + (size_t)pid * m.W);
-    uint32_t k = 0;
-    auto batch = [&](auto count) {
-        constexpr uint32_t N = decltype(count)::value;
-        int2 v[N / 2];
+// N entries of a pattern: their words, and the neighbours' components, all loads issued before the
+// first is used.
+template <typename R, uint32_t N>
+struct PatBatch {
+    int2 v[N / 2];
+    R x[N], y[N], z[N];
+    __device__ __forceinline__ void words(const int2* __restrict__ e) {
 #pragma unroll
-        for (uint32_t q = 0; q < N / 2; q++) v[q] = __ldg(e + k / 2 + q);
-        R x[N], y[N], z[N];
-        uint32_t t[N];
+        for (uint32_t q = 0; q < N / 2; q++) v[q] = __ldg(e + q);
+    }
+    __device__ __forceinline__ int32_t word(uint32_t q) const { return q & 1 ? v[q / 2].y : v[q / 2].x; }
+    __device__ __forceinline__ void spins(uint32_t i, const CVec3<R>& s) {
 #pragma unroll
         for (uint32_t q = 0; q < N; q++) {
-            const int32_t w = q & 1 ? v[q / 2].y : v[q / 2].x;
-            const uint32_t j = i + (uint32_t)(w >> 8);
-            t[q] = (uint32_t)w & 255u;
+            const uint32_t j = i + (uint32_t)(word(q) >> 8);
             x[q] = __ldg(s.p[0] + j); y[q] = __ldg(s.p[1] + j); z[q] = __ldg(s.p[2] + j);
         }
+    }
+    template <bool FULL>
+    __device__ __forceinline__ void add(const R* tab, R h[3]) const {
 #pragma unroll
-        for (uint32_t q = 0; q < N; q++) rs.add(tab, t[q], x[q], y[q], z[q], h);
-        k += N;
-    };
-    while (k + U <= m.W) batch(std::integral_constant<uint32_t, U>{});
-    while (k < m.W) batch(std::integral_constant<uint32_t, 2>{});
-    rs.finish(tab, h);
+        for (uint32_t q = 0; q < N; q++) accumulate_typed<R, FULL>(tab, (uint32_t)word(q) & 255u, x[q], y[q], z[q], h);
+    }
+};
+
+// h += sum over the row's pattern, from entry k on, of J_id S_{i + delta}; `tab` is the tensor table
+// (global memory for the diagonal form, whose few rows stay in L1; shared memory for full
+// tensors).
+template <typename R, bool FULL>
+__device__ __forceinline__ void gather_pattern(const PatDev& m, uint32_t pid, uint32_t i, const CVec3<R>& s,
+                                               const R* tab, R h[3], uint32_t k) {
+    const int2* __restrict__ e = reinterpret_cast<const int2*>(m.ent + (size_t)pid * m.W);
+    // (in FP64 six neighbours take 36 registers: 64×64×32 with dipole 39.7 → 45.7 µs per step)
+    if constexpr (sizeof(R) == 4) {
+        for (; k + PAT_BATCH <= m.W; k += PAT_BATCH) {
+            PatBatch<R, PAT_BATCH> b;
+            b.words(e + k / 2);
+            b.spins(i, s);
+            b.template add<FULL>(tab, h);
+        }
+    }
+#pragma unroll 3
+    for (; k < m.W; k += 2) {
+        PatBatch<R, 2> b;
+        b.words(e + k / 2);
+        b.spins(i, s);
+        b.template add<FULL>(tab, h);
+    }
 }
 
 // h += sum over diagonals d with 0 <= i+off[d] < n of J_{d,i} S_{i+off[d]}, row-aligned DIA.
@@ -304,7 +287,6 @@ __device__ __forceinline__ void gather_dia(const DiaDev& m, uint32_t n, uint32_t
     // the warp walks its tile's active diagonals (warp-uniform list)
     const uint32_t k0 = __ldg(m.tile_ptr + (i >> 5)), k1 = __ldg(m.tile_ptr + (i >> 5) + 1);
     if (m.dtype) {
-        RowSum<R, FULL> rs;
         for (uint32_t k = k0; k < k1; k++) {
             const uint32_t d = __ldg(m.tile_diag + k);
             const int64_t col = (int64_t)i + __ldg(m.off + d);
@@ -312,9 +294,8 @@ __device__ __forceinline__ void gather_dia(const DiaDev& m, uint32_t n, uint32_t
             const uint32_t t = ldcs(m.dtype + (size_t)d * n + i);
             if (t == 0) continue;
             const R x = __ldg(s.p[0] + col), y = __ldg(s.p[1] + col), z = __ldg(s.p[2] + col);
-            rs.add(tab, t, x, y, z, h);
+            accumulate_typed<R, FULL>(tab, t, x, y, z, h);
         }
-        rs.finish(tab, h);
         return;
     }
     const size_t ND = (size_t)m.ndiag * n;

@@ -61,8 +61,9 @@ struct PatDev {
 };
 constexpr int32_t PAT_DELTA = 1 << 23;  // |column - row| is below this
 constexpr uint32_t STAGE_PATTERN = 3;   // SellDev::stage: the stage kernels gather by row patterns
-// the stage kernel's layout parameter in that mode: at 48 registers, and at 64 (see MinBlocks)
-constexpr int EXCH_PATTERN = 4, EXCH_PATTERN_64 = 5;
+// the stage kernel's layout parameter in that mode: at 48 registers, at 64 (see MinBlocks), and at
+// 64 with the first neighbours loaded early (see stage_kernel)
+constexpr int EXCH_PATTERN = 4, EXCH_PATTERN_64 = 5, EXCH_PATTERN_EARLY = 6;
 constexpr uint32_t MAG_CHUNK = 2048;  // spins per block of the magnetisation reduction
 constexpr uint32_t SPIN_PAD = 8;     // zeroed elements after every gather-source spin array
 
