@@ -69,7 +69,7 @@ void free_all(asd_handle* h) {
         for (int q = 0; q < 6; q++) { F(h->kf[q][c]); F(h->kd[q][c]); }
     }
     if (h->h_err) cudaFreeHost(h->h_err);
-    F(h->d_err); F(h->d_aos); F(h->d_check); F(h->d_rep_of_tile); F(h->d_ttm); F(h->d_q4ptr); F(h->d_q4jkl);
+    F(h->d_err); F(h->d_gridbar); F(h->d_aos); F(h->d_check); F(h->d_rep_of_tile); F(h->d_ttm); F(h->d_q4ptr); F(h->d_q4jkl);
     F(h->pat.row); F(h->pat.ent);
     F(h->sell.lwords); F(h->sell.span_ptr); F(h->sell.spans);
     F(h->sell.slice_ptr); F(h->sell.a); F(h->sell.b); F(h->sell.c); F(h->sell.col); F(h->sell.val);
@@ -768,7 +768,7 @@ void build_graph(asd_handle* h, uint32_t steps) {
     h->step = 0;
     CK(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = cudaSuccess;
-    for (uint32_t r = 0; r < steps && e == cudaSuccess; r++) e = launch_fused_step(h, r, true);
+    e = launch_fused_steps(h, steps);
     if (e == cudaSuccess) e = launch_step_advance(h, steps);
     cudaError_t e2 = cudaStreamEndCapture(h->stream, &g);
     h->step = saved;
@@ -832,7 +832,7 @@ void run_steps(asd_handle* h, uint64_t nsteps) {
     const uint32_t G = h->graph_steps;
     uint64_t left = nsteps;
     auto direct = [&](uint64_t k) {
-        for (uint64_t r = 0; r < k; r++) CK(launch_fused_step(h, (uint32_t)r, false));
+        CK(launch_fused_steps(h, (uint32_t)k));
         CK(launch_step_advance(h, (uint32_t)k));
         h->step += k;
     };
@@ -1256,6 +1256,7 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
         CK(cudaEventCreate(&h->kev[0]));
         CK(cudaEventCreate(&h->kev[1]));
         h->d_err = dalloc<uint32_t>(1);
+        h->d_gridbar = dalloc<unsigned long long>(1);
         h->sell.err = h->d_err;
         CK(cudaHostAlloc(reinterpret_cast<void**>(&h->h_err), sizeof(uint32_t), cudaHostAllocDefault));
         if (!plain) {
@@ -1273,6 +1274,7 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
             if (G > 4096) G = upd;
             build_graph(h, G);
         }
+        CK(cudaStreamSynchronize(nullptr));               // the zeroing of the buffers above
         CK(cudaStreamSynchronize(h->stream));
     } catch (const Fail& f) {
         g_create_err = f.msg;
@@ -1501,6 +1503,12 @@ int asd_sync(asd_handle* h) {
         if (h->d_err) CK(cudaMemcpyAsync(h->h_err, h->d_err, sizeof e, cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
         if (h->d_err) e = *h->h_err;
+        if (e & 4u) {
+            CK(cudaMemset(h->d_err, 0, sizeof(uint32_t)));
+            CK(cudaMemset(h->d_gridbar, 0, sizeof(unsigned long long)));
+            CK(cudaStreamSynchronize(nullptr));           // before h->stream, which does not wait for it
+            throw Fail{ASD_ETIMEOUT, "a block's wait at the barrier between two stages ran out; the spins are invalid"};
+        }
         if (e & 2u) {
             CK(cudaMemset(h->d_err, 0, sizeof(uint32_t)));
             throw Fail{ASD_ETIMEOUT, "a long-range transform block's bulk-copy wait ran out; the long-range field of "

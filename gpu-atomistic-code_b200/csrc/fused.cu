@@ -130,147 +130,56 @@ constexpr uint32_t PATTERN_WAVE = 148 * 4 * 256;       // spins of one wave of 4
 template <int EX>
 constexpr bool is_pattern = EX == EXCH_PATTERN || EX == EXCH_PATTERN_64 || EX == EXCH_PATTERN_EARLY;
 
-// K: the stage kind at compile time (1 Heun predictor, 2 Heun corrector, 3 RK stage before the
-// last, 4 last RK stage); a.kind still carries the RK stage index.
-template <typename R, int EX, bool FULL, bool COMP, int K>
-__global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
-    stage_kernel(const StepConst c, const SellDev sell, const PatDev pat, const DiaDev dia, const StageArgs<R> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t stage_bar;
-    R* tab = reinterpret_cast<R*>(smem_raw);
-    // Until pdl_enter below the block touches only set-up data (the exchange words, the tensor
-    // table, the spans, the mesh index): the copies of the words and the table start while the
-    // previous kernel's last blocks run; the neighbour-spin spans are copied after the wait.
+template <typename R>
+__device__ __forceinline__ bool is_hot(const StepConst& c, uint32_t r) {
+    if constexpr (sizeof(R) == 4) return __ldg(c.rep_sqrtT_f + r) > 0.0f; else return __ldg(c.rep_sqrtT + r) > 0.0;
+}
+
+// The step's thermal field sigma sqrt(T) xi of spin i in replica r (T > 0).
+template <typename R>
+__device__ __forceinline__ void draw_thermal(const StepConst& c, const MatConst& mc, uint32_t r, uint32_t i, uint64_t t,
+                                             R lrn[3]) {
+    R xi[3], tp;
+    const uint32_t stream = __ldg(c.rep_stream + r), spin = i - __ldg(c.rep_off + r);
+    if constexpr (sizeof(R) == 4) {
+        thermal_normals_f(c.seed, stream, spin, t, xi);
+        tp = __ldg(c.rep_sqrtT_f + r) * mc.sigma_f;
+    } else {
+        thermal_normals(c.seed, stream, spin, t, xi);
+        tp = __ldg(c.rep_sqrtT + r) * mc.sigma;
+    }
+    for (int q = 0; q < 3; q++) lrn[q] = xi[q] * tp;
+}
+
+// What a row needs beside the arguments: the block's staged words, spins and table, and the row's
+// pattern with its first words.
+template <typename R>
+struct RowCtx {
     const uint32_t* staged = nullptr;
     const uint16_t* staged16 = nullptr;
     const R* sspin = nullptr;
-    R* span_dst = nullptr;           // shared-memory spin buffer the span copies fill after the wait
-    uint32_t span0 = 0, nspan = 0;
     uint32_t wbase = 0;
-    if constexpr (EX == ASD_EXCH_CSR) {
-        if (sell.typed) {
-            // the tensor table: with staging, one more bulk copy on the staging barrier; else a
-            // block-wide load
-            bool tab_staged = false;
-            const uint32_t tab_bytes = (uint32_t)sizeof(R) * table_stride<FULL>() * sell.ntypes;
-            if (sell.stage) {
-                // this block's slices are contiguous in the SELL stream: one bulk copy into
-                // shared memory behind the tensor table; with stage 2 also one copy per
-                // (neighbour-spin span, component); all overlap the noise draw below
-                const uint32_t tb = (tab_bytes + 15u) & ~15u;
-                const uint32_t spb = blockDim.x >> 5;
-                const uint32_t s0 = blockIdx.x * spb, s1 = min(s0 + spb, sell.nslices);
-                wbase = __ldg(sell.slice_ptr + s0);
-                const uint32_t bytes = (__ldg(sell.slice_ptr + s1) - wbase) * 4u;
-                uint32_t sp0 = 0, nsp = 0;
-                if (sell.stage == 2) {
-                    sp0 = __ldg(sell.span_ptr + blockIdx.x);
-                    nsp = __ldg(sell.span_ptr + blockIdx.x + 1) - sp0;
-                }
-                const bool w16 = sell.stage == 2 && sell.lwords16;
-                if (w16 && bytes && nsp) {
-                    // 16-bit local words (half the copy and the buffer) and the spans; a block
-                    // without spans stages nothing and reads its global words
-                    const uint32_t bytes16 = bytes >> 1;
-                    uint16_t* wbuf = reinterpret_cast<uint16_t*>(smem_raw + tb);
-                    R* sbuf = reinterpret_cast<R*>(smem_raw + tb + ((2u * sell.stage_words + 15u) & ~15u));
-                    if (threadIdx.x == 0) mbar_init(&stage_bar, 1);
-                    __syncthreads();
-                    if (threadIdx.x < 32) {
-                        if (threadIdx.x == 0) {
-                            uint32_t tx = bytes16 + tab_bytes;
-                            for (uint32_t q = 0; q < nsp; q++) tx += 3u * sell.spans[sp0 + q].y * (uint32_t)sizeof(R);
-                            mbar_arrive_expect_tx(&stage_bar, tx);
-                        }
-                        __syncwarp();
-                        if (threadIdx.x == 0) bulk_copy_stream(wbuf, sell.lwords16 + wbase, bytes16, &stage_bar);
-                        if (threadIdx.x == 1) bulk_copy(tab, table_of<R>(sell), tab_bytes, &stage_bar);
-                    }
-                    staged16 = wbuf;
-                    sspin = sbuf;
-                    span_dst = sbuf; span0 = sp0; nspan = nsp;
-                    tab_staged = true;
-                } else if (!w16 && bytes) {
-                    uint32_t* wbuf = reinterpret_cast<uint32_t*>(smem_raw + tb);
-                    R* sbuf = reinterpret_cast<R*>(smem_raw + tb + 4u * sell.stage_words);
-                    if (threadIdx.x == 0) mbar_init(&stage_bar, 1);
-                    __syncthreads();
-                    if (threadIdx.x < 32) {
-                        if (threadIdx.x == 0) {
-                            uint32_t tx = bytes + tab_bytes;
-                            for (uint32_t q = 0; q < nsp; q++) tx += 3u * sell.spans[sp0 + q].y * (uint32_t)sizeof(R);
-                            mbar_arrive_expect_tx(&stage_bar, tx);
-                        }
-                        __syncwarp();
-                        if (threadIdx.x == 0)
-                            bulk_copy_stream(wbuf, (nsp ? sell.lwords : sell.typed) + wbase, bytes, &stage_bar);
-                        if (threadIdx.x == 1) bulk_copy(tab, table_of<R>(sell), tab_bytes, &stage_bar);
-                    }
-                    staged = wbuf;
-                    if (nsp) { sspin = sbuf; span_dst = sbuf; span0 = sp0; nspan = nsp; }
-                    tab_staged = true;
-                }
-            }
-            if (!tab_staged) load_table<R>(table_of<R>(sell), table_stride<FULL>() * sell.ntypes, tab);
-        }
-    }
-    if constexpr (EX == ASD_EXCH_DIA) {
-        if (dia.dtype) load_table<R>(table_of<R>(dia), table_stride<FULL>() *dia.ntypes, tab);
-    }
-    // Row patterns (PatDev): no words to stage and no wait.  The stage reads 2 bytes of matrix per
-    // row instead of 28 (sc, 6 neighbours) or 108 (BCT-2, 26), and the pattern's entries come
-    // from L1, so all of the row's gathers are issued at once.  Measured against the fastest of the
-    // staged SELL shapes (step time in the graph, one B200): sc 128³ at 300 K 119.2 → 91.6 µs,
-    // 24 sc replicas (2.7 M spins) 155.0 → 121.6, sc 128×128×64 with dipole 175.9 → 163.0, BCT-2
-    // 64³ 55.4 → 49.2, sc 16³ 8.9 → 7.7.
-    // EARLY (FP32 lattices of at most one wave): the time of a stage is its chain of dependent loads,
-    // so the pattern's first words are read before the dependent-launch wait and their neighbours
-    // right after it, ahead of the thermal draw, and no L2 prefetch is issued (the state is in L2).
-    // µs per step: sc 16³ at 300 K 7.16 → 6.78, BCT-2 37×29×23 14.7 → 13.0; in FP64 (72 registers of
-    // neighbours held across the draw) it loses: 64×64×32 with dipole 45.7 → 47.6.
+    R* tab = nullptr;
+    uint64_t* bar = nullptr;
+    uint32_t pid = 0;
+    PatBatch<R, PAT_BATCH> first;
+    R lrn[3];                    // LIVE: the step's thermal field
+};
+
+// One stage of row i at step t.  K: the stage kind at compile time (1 Heun predictor, 2 Heun
+// corrector, 3 RK stage before the last, 4 last RK stage); a.kind still carries the RK stage
+// index.  LIVE: other blocks of the same launch write the spins it gathers.
+template <typename R, int EX, bool FULL, bool COMP, int K, bool LIVE>
+__device__ __forceinline__ void stage_row(const StepConst& c, const SellDev& sell, const PatDev& pat, const DiaDev& dia,
+                                          const StageArgs<R>& a, const uint32_t i, const uint64_t t, RowCtx<R>& x) {
     constexpr bool EARLY = EX == EXCH_PATTERN_EARLY;
     const bool early = EARLY && pat.W >= PAT_BATCH;
-    PatBatch<R, PAT_BATCH> first;
-    uint32_t pid = 0;
-    if constexpr (is_pattern<EX>) {
-        const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
-        if (row < c.n) pid = __ldg(pat.row + row);
-        if constexpr (EARLY)
-            if (early && row < c.n) first.words(reinterpret_cast<const int2*>(pat.ent + (size_t)pid * pat.W));
-        if constexpr (FULL) load_table<R>(table_of<R>(sell), table_stride<FULL>() * sell.ntypes, tab);
-        else tab = const_cast<R*>(table_of<R>(sell));
-    }
-    pdl_enter();
-    if constexpr (EX == ASD_EXCH_CSR) {
-        // the neighbour-spin spans: one copy per (span, component), on the staging barrier
-        if (threadIdx.x < 32)
-            for (uint32_t k = threadIdx.x; k < 3 * nspan; k += 32) {
-                const uint4 sp = sell.spans[span0 + k / 3];
-                const uint32_t cc = k % 3;
-                bulk_copy(span_dst + cc * sell.spin_slots + sp.z, a.src.p[cc] + sp.x, sp.y * (uint32_t)sizeof(R),
-                          &stage_bar);
-            }
-    }
-    if (!EARLY && threadIdx.x == 0 && a.npf) {
-        // the block's rows of every per-spin input: one bulk L2 prefetch each, so the loads
-        // after the exchange gather find them in L2; sizes stop at the last row (whole
-        // 16-byte units), so no prefetch reaches past an array
-        const uint32_t r0 = blockIdx.x * blockDim.x;
-        const uint32_t rows = min(blockDim.x, c.n - r0);
-        const uint32_t bytes = (rows * (uint32_t)sizeof(R)) & ~15u;
-        if (bytes)
-            for (uint32_t q = 0; q < a.npf; q++)
-                bulk_prefetch_l2(static_cast<const char*>(a.pf[q]) + (size_t)r0 * sizeof(R), bytes);
-    }
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= c.n) return;     // thread 0 of every block has i < n and always waits below
     // stage spin at this site; the pattern kernels load it with the gather's first loads
     R sv[3];
     if constexpr (EARLY) {
         for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
-        if (early) first.spins(i, a.src);
+        if (early) x.first.template spins<LIVE>(i, a.src);
     }
-    const uint64_t t = *c.step_base + a.rel;
     const uint32_t at = atom_of(c, i);
     const MatConst& mc = c.mat[at];
     const uint32_t r = replica_of(c, i);
@@ -278,22 +187,12 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
     // one thermal draw per spin and step serves every stage (src/cuint.cu:72): the first stage
     // draws it, later stages of the step load what the first stored
     R lrn[3] = {R(0), R(0), R(0)};
-    bool hot;
-    if constexpr (F32) hot = __ldg(c.rep_sqrtT_f + r) > 0.0f; else hot = __ldg(c.rep_sqrtT + r) > 0.0;
-    if (hot && a.nz_mode == 2) {
-        lrn[0] = a.nz.p[0][i]; lrn[1] = a.nz.p[1][i]; lrn[2] = a.nz.p[2][i];
-    } else if (hot) {
-        if constexpr (F32) {
-            float xi[3];
-            thermal_normals_f(c.seed, __ldg(c.rep_stream + r), i - __ldg(c.rep_off + r), t, xi);
-            const float tp = __ldg(c.rep_sqrtT_f + r) * mc.sigma_f;
-            lrn[0] = xi[0] * tp; lrn[1] = xi[1] * tp; lrn[2] = xi[2] * tp;
-        } else {
-            double xi[3];
-            thermal_normals(c.seed, __ldg(c.rep_stream + r), i - __ldg(c.rep_off + r), t, xi);
-            const double tp = __ldg(c.rep_sqrtT + r) * mc.sigma;
-            lrn[0] = xi[0] * tp; lrn[1] = xi[1] * tp; lrn[2] = xi[2] * tp;
-        }
+    if constexpr (LIVE) {
+        for (int q = 0; q < 3; q++) lrn[q] = x.lrn[q];    // drawn behind the barrier before the step
+    } else if (a.nz_mode == 2) {
+        if (is_hot<R>(c, r)) { lrn[0] = a.nz.p[0][i]; lrn[1] = a.nz.p[1][i]; lrn[2] = a.nz.p[2][i]; }
+    } else if (is_hot<R>(c, r)) {
+        draw_thermal<R>(c, mc, r, i, t, lrn);
         if (a.nz_mode == 1) { a.nz.p[0][i] = lrn[0]; a.nz.p[1][i] = lrn[1]; a.nz.p[2][i] = lrn[2]; }
     }
     // the long-range field at this site: with diagonal tensors it is loaded before the staging
@@ -312,24 +211,24 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
     if constexpr (!FULL) load_lr();
     bool stage_timeout = false;
     const uint32_t polls = (c.flags & ASD_FLAG_WAIT_TIMEOUT) ? 0u : STAGE_WAIT_POLLS;
-    if ((staged || staged16) && !mbar_wait_bounded(&stage_bar, polls)) {
+    if ((x.staged || x.staged16) && !mbar_wait_bounded(x.bar, polls)) {
         // the copy did not land in time: record it and read the words and the table from
         // global memory
         atomicOr(sell.err, ERR_STAGE_TIMEOUT);
-        staged = nullptr;      // the global words carry global columns
-        staged16 = nullptr;
-        sspin = nullptr;
-        tab = const_cast<R*>(table_of<R>(sell));
+        x.staged = nullptr;    // the global words carry global columns
+        x.staged16 = nullptr;
+        x.sspin = nullptr;
+        x.tab = const_cast<R*>(table_of<R>(sell));
         stage_timeout = true;
     }
     R h[3] = {R(0), R(0), R(0)};
     if constexpr (is_pattern<EX> && !EARLY)
         for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
-    if constexpr (EX == ASD_EXCH_CSR) gather_sell<R, FULL>(sell, i, a.src, tab, h, staged, wbase, sspin, staged16);
-    if constexpr (EX == ASD_EXCH_DIA) gather_dia<R, FULL>(dia, c.n, i, a.src, tab, h);
+    if constexpr (EX == ASD_EXCH_CSR) gather_sell<R, FULL>(sell, i, a.src, x.tab, h, x.staged, x.wbase, x.sspin, x.staged16);
+    if constexpr (EX == ASD_EXCH_DIA) gather_dia<R, FULL>(dia, c.n, i, a.src, x.tab, h);
     if constexpr (is_pattern<EX>) {
-        if (early) first.template add<FULL>(tab, h);
-        gather_pattern<R, FULL>(pat, pid, i, a.src, tab, h, early ? PAT_BATCH : 0u);
+        if (early) x.first.template add<FULL>(x.tab, h);
+        gather_pattern<R, FULL, LIVE>(pat, x.pid, i, a.src, x.tab, h, early ? PAT_BATCH : 0u);
     }
     if (c.q4_ptr) {
         R h4[3];
@@ -450,7 +349,230 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
         a.lr.mr[2 * a.lr.P + midx] = (float)out[2] * wv;
     }
     // a block must not retire while its bulk copy may still be writing shared memory
-    if (stage_timeout) mbar_wait_bounded(&stage_bar, STAGE_WAIT_POLLS);
+    if (stage_timeout) mbar_wait_bounded(x.bar, STAGE_WAIT_POLLS);
+}
+
+template <typename R, int EX, bool FULL, bool COMP, int K>
+__global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
+    stage_kernel(const StepConst c, const SellDev sell, const PatDev pat, const DiaDev dia, const StageArgs<R> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(8) uint64_t stage_bar;
+    R* tab = reinterpret_cast<R*>(smem_raw);
+    // Until pdl_enter below the block touches only set-up data (the exchange words, the tensor
+    // table, the spans, the mesh index): the copies of the words and the table start while the
+    // previous kernel's last blocks run; the neighbour-spin spans are copied after the wait.
+    RowCtx<R> x;
+    x.bar = &stage_bar;
+    R* span_dst = nullptr;           // shared-memory spin buffer the span copies fill after the wait
+    uint32_t span0 = 0, nspan = 0;
+    uint32_t& wbase = x.wbase;
+    if constexpr (EX == ASD_EXCH_CSR) {
+        if (sell.typed) {
+            // the tensor table: with staging, one more bulk copy on the staging barrier; else a
+            // block-wide load
+            bool tab_staged = false;
+            const uint32_t tab_bytes = (uint32_t)sizeof(R) * table_stride<FULL>() * sell.ntypes;
+            if (sell.stage) {
+                // this block's slices are contiguous in the SELL stream: one bulk copy into
+                // shared memory behind the tensor table; with stage 2 also one copy per
+                // (neighbour-spin span, component); all overlap the noise draw below
+                const uint32_t tb = (tab_bytes + 15u) & ~15u;
+                const uint32_t spb = blockDim.x >> 5;
+                const uint32_t s0 = blockIdx.x * spb, s1 = min(s0 + spb, sell.nslices);
+                wbase = __ldg(sell.slice_ptr + s0);
+                const uint32_t bytes = (__ldg(sell.slice_ptr + s1) - wbase) * 4u;
+                uint32_t sp0 = 0, nsp = 0;
+                if (sell.stage == 2) {
+                    sp0 = __ldg(sell.span_ptr + blockIdx.x);
+                    nsp = __ldg(sell.span_ptr + blockIdx.x + 1) - sp0;
+                }
+                const bool w16 = sell.stage == 2 && sell.lwords16;
+                if (w16 && bytes && nsp) {
+                    // 16-bit local words (half the copy and the buffer) and the spans; a block
+                    // without spans stages nothing and reads its global words
+                    const uint32_t bytes16 = bytes >> 1;
+                    uint16_t* wbuf = reinterpret_cast<uint16_t*>(smem_raw + tb);
+                    R* sbuf = reinterpret_cast<R*>(smem_raw + tb + ((2u * sell.stage_words + 15u) & ~15u));
+                    if (threadIdx.x == 0) mbar_init(&stage_bar, 1);
+                    __syncthreads();
+                    if (threadIdx.x < 32) {
+                        if (threadIdx.x == 0) {
+                            uint32_t tx = bytes16 + tab_bytes;
+                            for (uint32_t q = 0; q < nsp; q++) tx += 3u * sell.spans[sp0 + q].y * (uint32_t)sizeof(R);
+                            mbar_arrive_expect_tx(&stage_bar, tx);
+                        }
+                        __syncwarp();
+                        if (threadIdx.x == 0) bulk_copy_stream(wbuf, sell.lwords16 + wbase, bytes16, &stage_bar);
+                        if (threadIdx.x == 1) bulk_copy(tab, table_of<R>(sell), tab_bytes, &stage_bar);
+                    }
+                    x.staged16 = wbuf;
+                    x.sspin = sbuf;
+                    span_dst = sbuf; span0 = sp0; nspan = nsp;
+                    tab_staged = true;
+                } else if (!w16 && bytes) {
+                    uint32_t* wbuf = reinterpret_cast<uint32_t*>(smem_raw + tb);
+                    R* sbuf = reinterpret_cast<R*>(smem_raw + tb + 4u * sell.stage_words);
+                    if (threadIdx.x == 0) mbar_init(&stage_bar, 1);
+                    __syncthreads();
+                    if (threadIdx.x < 32) {
+                        if (threadIdx.x == 0) {
+                            uint32_t tx = bytes + tab_bytes;
+                            for (uint32_t q = 0; q < nsp; q++) tx += 3u * sell.spans[sp0 + q].y * (uint32_t)sizeof(R);
+                            mbar_arrive_expect_tx(&stage_bar, tx);
+                        }
+                        __syncwarp();
+                        if (threadIdx.x == 0)
+                            bulk_copy_stream(wbuf, (nsp ? sell.lwords : sell.typed) + wbase, bytes, &stage_bar);
+                        if (threadIdx.x == 1) bulk_copy(tab, table_of<R>(sell), tab_bytes, &stage_bar);
+                    }
+                    x.staged = wbuf;
+                    if (nsp) { x.sspin = sbuf; span_dst = sbuf; span0 = sp0; nspan = nsp; }
+                    tab_staged = true;
+                }
+            }
+            if (!tab_staged) load_table<R>(table_of<R>(sell), table_stride<FULL>() * sell.ntypes, tab);
+        }
+    }
+    if constexpr (EX == ASD_EXCH_DIA) {
+        if (dia.dtype) load_table<R>(table_of<R>(dia), table_stride<FULL>() *dia.ntypes, tab);
+    }
+    // Row patterns (PatDev): no words to stage and no wait.  The stage reads 2 bytes of matrix per
+    // row instead of 28 (sc, 6 neighbours) or 108 (BCT-2, 26), and the pattern's entries come
+    // from L1, so all of the row's gathers are issued at once.  Measured against the fastest of the
+    // staged SELL shapes (step time in the graph, one B200): sc 128³ at 300 K 119.2 → 91.6 µs,
+    // 24 sc replicas (2.7 M spins) 155.0 → 121.6, sc 128×128×64 with dipole 175.9 → 163.0, BCT-2
+    // 64³ 55.4 → 49.2, sc 16³ 8.9 → 7.7.
+    // EARLY (FP32 lattices of at most one wave): the time of a stage is its chain of dependent loads,
+    // so the pattern's first words are read before the dependent-launch wait and their neighbours
+    // right after it, ahead of the thermal draw, and no L2 prefetch is issued (the state is in L2).
+    // µs per step: sc 16³ at 300 K 7.16 → 6.78, BCT-2 37×29×23 14.7 → 13.0; in FP64 (72 registers of
+    // neighbours held across the draw) it loses: 64×64×32 with dipole 45.7 → 47.6.
+    constexpr bool EARLY = EX == EXCH_PATTERN_EARLY;
+    const bool early = EARLY && pat.W >= PAT_BATCH;
+    if constexpr (is_pattern<EX>) {
+        const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
+        if (row < c.n) x.pid = __ldg(pat.row + row);
+        if constexpr (EARLY)
+            if (early && row < c.n) x.first.words(reinterpret_cast<const int2*>(pat.ent + (size_t)x.pid * pat.W));
+        if constexpr (FULL) load_table<R>(table_of<R>(sell), table_stride<FULL>() * sell.ntypes, tab);
+        else tab = const_cast<R*>(table_of<R>(sell));
+    }
+    pdl_enter();
+    if constexpr (EX == ASD_EXCH_CSR) {
+        // the neighbour-spin spans: one copy per (span, component), on the staging barrier
+        if (threadIdx.x < 32)
+            for (uint32_t k = threadIdx.x; k < 3 * nspan; k += 32) {
+                const uint4 sp = sell.spans[span0 + k / 3];
+                const uint32_t cc = k % 3;
+                bulk_copy(span_dst + cc * sell.spin_slots + sp.z, a.src.p[cc] + sp.x, sp.y * (uint32_t)sizeof(R),
+                          &stage_bar);
+            }
+    }
+    if (!EARLY && threadIdx.x == 0 && a.npf) {
+        // the block's rows of every per-spin input: one bulk L2 prefetch each, so the loads
+        // after the exchange gather find them in L2; sizes stop at the last row (whole
+        // 16-byte units), so no prefetch reaches past an array
+        const uint32_t r0 = blockIdx.x * blockDim.x;
+        const uint32_t rows = min(blockDim.x, c.n - r0);
+        const uint32_t bytes = (rows * (uint32_t)sizeof(R)) & ~15u;
+        if (bytes)
+            for (uint32_t q = 0; q < a.npf; q++)
+                bulk_prefetch_l2(static_cast<const char*>(a.pf[q]) + (size_t)r0 * sizeof(R), bytes);
+    }
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= c.n) return;     // thread 0 of every block has i < n and always waits below
+    x.tab = tab;
+    stage_row<R, EX, FULL, COMP, K, false>(c, sell, pat, dia, a, i, *c.step_base + a.rel, x);
+}
+
+// ---- several steps in one launch (small lattices) ----
+// Below about two blocks per SM a stage is not bound by its work but by the way from one launch to
+// the next: the grid's drain, the dependent launch, and a first round trip to L2 for everything
+// the last launch left in its L1 and registers.  Here one cooperative launch runs `nsteps` steps: each
+// thread keeps its row, its pattern, the constants and the step's thermal field (drawn for the next step
+// between arriving at the barrier and waiting there, 6.28 → 5.87 µs per step on sc 16³ together
+// with neighbours through L1), and a barrier over the grid (a counter in L2, waits bounded) stands
+// between the stages.
+constexpr uint32_t MAX_STAGES = 6;
+constexpr uint32_t ERR_RESIDENT_TIMEOUT = 4u;
+constexpr uint32_t RESIDENT_WAIT_POLLS = 1u << 21;     // about a second
+
+template <typename R>
+struct ResidentArgs {
+    StageArgs<R> st[MAX_STAGES];
+    uint32_t nst;                // stages per step (2: Heun)
+    uint32_t nsteps;
+    unsigned long long* barrier; // arrivals so far: a multiple of the grid between launches
+    uint32_t* err;
+};
+
+// The barrier in two halves: every block arrives once its stores are done, and waits until all have
+// (their stores are then visible); false when the wait ran out.  In between goes what does not
+// depend on the other blocks.
+__device__ __forceinline__ void barrier_arrive(unsigned long long* arrivals, unsigned long long& target) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        const unsigned long long v = atomicAdd(arrivals, 1ull) + 1;
+        if (target == 0) target = (v + gridDim.x - 1) / gridDim.x * gridDim.x;   // this launch's first barrier
+        else target += gridDim.x;
+    }
+}
+__device__ __forceinline__ bool barrier_wait(unsigned long long* arrivals, unsigned long long target, uint32_t* err) {
+    __shared__ uint32_t ok;
+    if (threadIdx.x == 0) {
+        unsigned long long v = 0;
+        uint32_t it = 0;
+        do asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(arrivals) : "memory");
+        while (v < target && ++it < RESIDENT_WAIT_POLLS);
+        asm volatile("fence.acq_rel.gpu;" ::: "memory");
+        ok = v >= target;
+        if (v < target) atomicOr(err, ERR_RESIDENT_TIMEOUT);
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+template <typename R, bool FULL, bool COMP, bool HEUN>
+__global__ void __launch_bounds__(256, 2)
+    resident_kernel(const StepConst c, const SellDev sell, const PatDev pat, const ResidentArgs<R> ra) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    RowCtx<R> x;
+    x.tab = reinterpret_cast<R*>(smem_raw);
+    load_table<R>(table_of<R>(sell), table_stride<FULL>() * sell.ntypes, x.tab);
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool row = i < c.n;
+    const uint64_t t0 = *c.step_base;
+    uint32_t rep = 0;
+    bool hot = false;
+    x.lrn[0] = x.lrn[1] = x.lrn[2] = R(0);
+    if (row) {
+        x.pid = __ldg(pat.row + i);
+        if (pat.W >= PAT_BATCH) x.first.words(reinterpret_cast<const int2*>(pat.ent + (size_t)x.pid * pat.W));
+        rep = replica_of(c, i);
+        hot = is_hot<R>(c, rep);
+        if (hot) draw_thermal<R>(c, c.mat[atom_of(c, i)], rep, i, t0, x.lrn);
+    }
+    const DiaDev none{};
+    unsigned long long target = 0;
+    for (uint32_t s = 0; s < ra.nsteps; s++)
+        for (uint32_t q = 0; q < ra.nst; q++) {
+            const bool last = q + 1 == ra.nst;
+            if (row) {
+                constexpr int EX = EXCH_PATTERN_EARLY;
+                if constexpr (HEUN) {
+                    if (q == 0) stage_row<R, EX, FULL, COMP, 1, true>(c, sell, pat, none, ra.st[0], i, t0 + s, x);
+                    else stage_row<R, EX, FULL, COMP, 2, true>(c, sell, pat, none, ra.st[1], i, t0 + s, x);
+                } else {
+                    if (!last) stage_row<R, EX, FULL, COMP, 3, true>(c, sell, pat, none, ra.st[q], i, t0 + s, x);
+                    else stage_row<R, EX, FULL, COMP, 4, true>(c, sell, pat, none, ra.st[q], i, t0 + s, x);
+                }
+            }
+            if (last && s + 1 == ra.nsteps) return;
+            barrier_arrive(ra.barrier, target);
+            if (last && hot) draw_thermal<R>(c, c.mat[atom_of(c, i)], rep, i, t0 + s + 1, x.lrn);
+            if (!barrier_wait(ra.barrier, target, ra.err)) return;
+        }
 }
 
 __global__ void advance_k(uint64_t* step, uint32_t n) {
@@ -601,6 +723,71 @@ void set_prefetch(StageArgs<R>& a, bool comp) {
     a.npf = k;
 }
 
+// Spins up to which the steps of a pattern matrix run as one cooperative launch: two blocks of 256 per
+// SM, full tensors one of 128.  Measured against one launch per stage (µs per step in 32-step chunks,
+// one B200): sc 8³ 6.44 → 4.91, 16³ at 300 K 6.78 → 5.87, 40³ 7.28 → 6.51, 64³ 15.4 → 15.6; BCT-2
+// 6×7×6 cells 9.19 → 7.92, 20³ 10.1 → 9.2, 37×29×23 13.0 → 13.5.
+constexpr uint32_t RESIDENT_MAX = 148 * 2 * 256, RESIDENT_MAX_FULL = 148 * 128;
+
+template <typename R, bool FULL, bool COMP, bool HEUN>
+cudaError_t launch_resident_k(asd_handle* h, const ResidentArgs<R>& ra) {
+    const void* kern = reinterpret_cast<const void*>(resident_kernel<R, FULL, COMP, HEUN>);
+    // the smallest blocks that leave no SM two of them
+    const uint32_t block = h->n <= 148 * 64 ? 64 : h->n <= 148 * 128 ? 128 : 256;
+    const uint32_t grid = (h->n + block - 1) / block;
+    const size_t smem = sizeof(R) * table_stride<FULL>() * h->sell.ntypes;
+    uint32_t most = 0;
+    cudaError_t e = resident_grid(kern, block, smem, grid, &most);
+    if (e != cudaSuccess) return e;
+    if (most < grid) return cudaErrorCooperativeLaunchTooLarge;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if ((e = cudaLaunchKernelEx(&cfg, resident_kernel<R, FULL, COMP, HEUN>, h->sc, h->sell, h->pat, ra)) != cudaSuccess)
+        return e;
+    h->launches += 1;
+    return cudaGetLastError();
+}
+
+template <bool COMP, bool HEUN>
+cudaError_t launch_resident(asd_handle* h, const ResidentArgs<float>& ra) {
+    return h->full ? launch_resident_k<float, true, COMP, HEUN>(h, ra) : launch_resident_k<float, false, COMP, HEUN>(h, ra);
+}
+
+// The stages of one step without a long-range field, as fused_step_t launches them.
+ResidentArgs<float> resident_args(asd_handle* h, bool comp) {
+    ResidentArgs<float> ra{};
+    const bool heun = h->p.integrator == ASD_HEUN;
+    ra.nst = heun ? 2 : h->p.integrator == ASD_RK4 ? 4 : 6;
+    float* const* pp[2] = {h->esf, h->fnf};
+    for (uint32_t q = 0; q < ra.nst; q++) {
+        StageArgs<float>& a = ra.st[q];
+        const bool last = q + 1 == ra.nst;
+        a.base = c3<float>(h->sf);
+        if (comp) a.base_lo = CVec3<float>{{h->sl[0], h->sl[1], h->sl[2]}};
+        if (h->stagf[0]) a.stag = c3<float>(h->stagf);
+        a.nz = v3<float>(h->nzf);
+        a.nz_mode = q == 0 ? 1 : 2;
+        a.nst = heun ? 0 : (int)ra.nst;
+        a.kind = heun ? 1 + (int)q : 10 + (int)q;
+        a.src = q == 0 ? c3<float>(h->sf) : c3<float>(heun ? h->esf : pp[(q - 1) & 1]);
+        a.out = last ? v3<float>(h->sf) : v3<float>(heun ? h->esf : pp[q & 1]);
+        if (comp && last) a.out_lo = Vec3<float>{{h->sl[0], h->sl[1], h->sl[2]}};
+        if (heun) { a.fn = v3<float>(h->fnf); a.det = v3<float>(h->detf); }
+        else for (int b = 0; b < 6; b++) a.k[b] = v3<float>(h->kf[b]);
+    }
+    ra.barrier = h->d_gridbar;
+    ra.err = h->d_err;
+    return ra;
+}
+
 template <typename R>
 cudaError_t fused_step_t(asd_handle* h, uint32_t rel) {
     R* const* s; R* const* es; R* const* fn; R* const* det; R* const* stag;
@@ -734,6 +921,28 @@ cudaError_t time_first_stage(asd_handle* h, int warm, int reps, float* ms) {
 cudaError_t launch_fused_step(asd_handle* h, uint32_t rel, bool) {
     if (h->p.precision == ASD_FP32) return fused_step_t<float>(h, rel);
     return fused_step_t<double>(h, rel);
+}
+
+// Steps rel = 0 .. k-1 from the device step counter (phase h->step): one cooperative launch where the
+// lattice is small, its matrix has patterns and nothing else runs between the stages; else step by step.
+cudaError_t launch_fused_steps(asd_handle* h, uint32_t k) {
+    const bool one = k > 1 && h->n <= (h->full ? RESIDENT_MAX_FULL : RESIDENT_MAX) && h->p.precision == ASD_FP32 && h->dexch == ASD_EXCH_CSR &&
+                     h->sell.stage == STAGE_PATTERN && h->lr.mode == ASD_LR_NONE && !h->d_ttm && !h->sc.q4_ptr && step_pdl(h) &&
+                     !(h->p.flags & ASD_FLAG_WAIT_TIMEOUT);
+    if (one) {
+        const bool comp = (h->p.flags & ASD_FLAG_COMPENSATED) != 0, heun = h->p.integrator == ASD_HEUN;
+        ResidentArgs<float> ra = resident_args(h, comp);
+        ra.nsteps = k;
+        const cudaError_t e = comp ? (heun ? launch_resident<true, true>(h, ra) : launch_resident<true, false>(h, ra))
+                                   : (heun ? launch_resident<false, true>(h, ra) : launch_resident<false, false>(h, ra));
+        if (e != cudaErrorCooperativeLaunchTooLarge) return e;
+        cudaGetLastError();
+    }
+    for (uint32_t r = 0; r < k; r++) {
+        const cudaError_t e = launch_fused_step(h, r, false);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 cudaError_t launch_det_here(asd_handle* h) {

@@ -241,11 +241,15 @@ struct PatBatch {
         for (uint32_t q = 0; q < N / 2; q++) v[q] = __ldg(e + q);
     }
     __device__ __forceinline__ int32_t word(uint32_t q) const { return q & 1 ? v[q / 2].y : v[q / 2].x; }
+    // LIVE: other blocks of this launch write the spins, ordered by its barriers: ordinary loads, not
+    // the read-only path's
+    template <bool LIVE>
     __device__ __forceinline__ void spins(uint32_t i, const CVec3<R>& s) {
 #pragma unroll
         for (uint32_t q = 0; q < N; q++) {
             const uint32_t j = i + (uint32_t)(word(q) >> 8);
-            x[q] = __ldg(s.p[0] + j); y[q] = __ldg(s.p[1] + j); z[q] = __ldg(s.p[2] + j);
+            if constexpr (LIVE) { x[q] = s.p[0][j]; y[q] = s.p[1][j]; z[q] = s.p[2][j]; }
+            else { x[q] = __ldg(s.p[0] + j); y[q] = __ldg(s.p[1] + j); z[q] = __ldg(s.p[2] + j); }
         }
     }
     template <bool FULL>
@@ -258,7 +262,7 @@ struct PatBatch {
 // h += sum over the row's pattern, from entry k on, of J_id S_{i + delta}; `tab` is the tensor table
 // (global memory for the diagonal form, whose few rows stay in L1; shared memory for full
 // tensors).
-template <typename R, bool FULL>
+template <typename R, bool FULL, bool LIVE>
 __device__ __forceinline__ void gather_pattern(const PatDev& m, uint32_t pid, uint32_t i, const CVec3<R>& s,
                                                const R* tab, R h[3], uint32_t k) {
     const int2* __restrict__ e = reinterpret_cast<const int2*>(m.ent + (size_t)pid * m.W);
@@ -267,7 +271,7 @@ __device__ __forceinline__ void gather_pattern(const PatDev& m, uint32_t pid, ui
         for (; k + PAT_BATCH <= m.W; k += PAT_BATCH) {
             PatBatch<R, PAT_BATCH> b;
             b.words(e + k / 2);
-            b.spins(i, s);
+            b.template spins<LIVE>(i, s);
             b.template add<FULL>(tab, h);
         }
     }
@@ -275,7 +279,7 @@ __device__ __forceinline__ void gather_pattern(const PatDev& m, uint32_t pid, ui
     for (; k < m.W; k += 2) {
         PatBatch<R, 2> b;
         b.words(e + k / 2);
-        b.spins(i, s);
+        b.template spins<LIVE>(i, s);
         b.template add<FULL>(tab, h);
     }
 }

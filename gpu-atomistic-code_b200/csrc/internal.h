@@ -211,7 +211,8 @@ struct asd_handle {
     uint64_t graph_launches = 0;
     std::vector<uint32_t> h_slice_ptr;   // SELL slice offsets (host copy, for staging capacity)
     std::vector<uint32_t> h_words;       // typed SELL words (host copy, for the local words)
-    uint32_t* d_err = nullptr;           // device error bits (staging wait timeouts)
+    uint32_t* d_err = nullptr;           // device error bits (waits that ran out)
+    unsigned long long* d_gridbar = nullptr; // arrivals at the grid barrier of the several-steps kernel
     uint32_t* h_err = nullptr;           // page-locked host word the error bits are read into
     double* d_aos = nullptr;             // [3N] staging buffer of the spin / field transfers
     unsigned long long* d_check = nullptr; // [2] first non-finite component, first zero-length spin
@@ -281,6 +282,7 @@ namespace asd {
 // launchers implemented in the .cu files; all return cudaError_t of the launch
 cudaError_t launch_plain_step(asd_handle* h, uint64_t t);
 cudaError_t launch_fused_step(asd_handle* h, uint32_t rel, bool in_capture);
+cudaError_t launch_fused_steps(asd_handle* h, uint32_t k);
 cudaError_t launch_step_advance(asd_handle* h, uint32_t nsteps);
 cudaError_t launch_det_here(asd_handle* h);
 // The one-step graph's det_here_k node with the applied field h->p.applied (no launch).
