@@ -446,37 +446,20 @@ void setup_lr(asd_handle* h, const asd_system& s, bool plain) {
         for (auto& pr : pairs)
             if (std::fabs(s.nr[pr[0] * L.P + c] - s.nr[pr[1] * L.P + c]) > 1e-13 * amax) sym = false;
     L.ncomp = sym ? 6 : 9;
-    std::vector<double> nrs(s.nr, s.nr + 9 * L.P);
-    if (sym)
-        for (size_t c = 0; c < L.P; c++)
-            for (auto& pr : pairs) {
-                const double m = 0.5 * (nrs[pr[0] * L.P + c] + nrs[pr[1] * L.P + c]);
-                nrs[pr[0] * L.P + c] = m;
-                nrs[pr[1] * L.P + c] = m;
-            }
     uint32_t lo[3] = {~0u, ~0u, ~0u}, hi[3] = {0, 0, 0};    // bounding box of the spins on the mesh
     for (uint32_t i = 0; i < h->n; i++)
         for (int a = 0; a < 3; a++) {
             lo[a] = std::min(lo[a], s.mesh_xyz[3 * i + a]);
             hi[a] = std::max(hi[a], s.mesh_xyz[3 * i + a]);
         }
-    if (!plain) {
-        // On an even mesh axis the plane at index m/2 holds the aliased displacement +-m/2; when
-        // the spins span fewer than m/2 mesh points along that axis no two spins are that far
-        // apart, so the plane never reaches a spin and is cleared.  N_r is then exactly even
-        // (N(-r) = N(r)), its transform real, and the convolution takes the 6-component real form.
-        for (int a = 0; a < 3; a++) {
-            const uint32_t m = L.mesh[a];
-            if (m % 2 || h->n == 0 || hi[a] - lo[a] >= m / 2) continue;
-            for (uint32_t x = 0; x < L.mesh[0]; x++)
-                for (uint32_t y = 0; y < L.mesh[1]; y++)
-                    for (uint32_t z = 0; z < L.mesh[2]; z++) {
-                        const uint32_t v[3] = {x, y, z};
-                        if (v[a] != m / 2) continue;
-                        const size_t c = ((size_t)x * L.mesh[1] + y) * L.mesh[2] + z;
-                        for (int q = 0; q < 9; q++) nrs[q * L.P + c] = 0.0;
-                    }
-        }
+    // On an even mesh axis the plane at index m/2 holds the aliased displacement +-m/2; when
+    // the spins span fewer than m/2 mesh points along that axis no two spins are that far
+    // apart, so the plane never reaches a spin and is cleared (prepare_nr).  N_r is then exactly even
+    // (N(-r) = N(r)), its transform real, and the convolution takes the 6-component real form.
+    uint32_t clear = 0;
+    for (int a = 0; a < 3; a++) {
+        const uint32_t m = L.mesh[a];
+        if (m % 2 == 0 && h->n > 0 && hi[a] - lo[a] < m / 2) clear |= 1u << a;
     }
     // The plane kernels where their axis lengths, the box and the shared memory fit; a complex N_k
     // must fit as well unless N_r is even over the box (then N_k is real).
@@ -495,7 +478,7 @@ void setup_lr(asd_handle* h, const asd_system& s, bool plain) {
                         mir = mir * s.mesh[a] + (c[a] ? s.mesh[a] - c[a] : 0);
                     }
                     for (int q = 0; q < 9; q++)
-                        if (std::fabs(nrs[q * L.P + at] - nrs[q * L.P + mir]) > 1e-13 * amax) return false;
+                        if (std::fabs(s.nr[q * L.P + at] - s.nr[q * L.P + mir]) > 1e-13 * amax) return false;
                 }
         return true;
     };
@@ -540,7 +523,16 @@ void setup_lr(asd_handle* h, const asd_system& s, bool plain) {
                                 (s.mesh_xyz[3 * i + 2] - org[2]));
         L.mesh_idx = dupload(idx.data(), idx.size());
     }
-    double* d_nr = dupload(plain ? s.nr : nrs.data(), nrs.size());
+    const size_t P_in = (size_t)s.mesh[0] * s.mesh[1] * s.mesh[2];
+    double* d_nr = dupload(s.nr, 9 * P_in);
+    if (!plain) {
+        CK(cudaStreamSynchronize(nullptr));                // the upload, which h->stream does not wait for
+        const cudaError_t ep = prepare_nr(h, s.mesh, clear, sym, d_nr);
+        if (ep != cudaSuccess) {
+            cudaFree(d_nr);
+            CK(ep);
+        }
+    }
     if (moved) {
         // (not dalloc: its zeroing runs on the default stream, which h->stream does not wait for;
         // embed_nr zeroes on h->stream)

@@ -652,6 +652,23 @@ __global__ void nk_parity_x(size_t Pk, uint32_t m0, uint32_t m1, uint32_t Kz, co
     }
 }
 
+__global__ void prepare_nr_k(uint3 m, uint32_t clear, int sym, double* __restrict__ nr) {
+    const size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x, P = (size_t)m.x * m.y * m.z;
+    if (c >= P) return;
+    const uint32_t z = (uint32_t)(c % m.z), y = (uint32_t)(c / m.z % m.y), x = (uint32_t)(c / m.z / m.y);
+    if (((clear & 1u) && x == m.x / 2) || ((clear & 2u) && y == m.y / 2) || ((clear & 4u) && z == m.z / 2)) {
+        for (int q = 0; q < 9; q++) nr[q * P + c] = 0.0;
+    } else if (sym) {
+        constexpr int pairs[3][2] = {{1, 3}, {2, 6}, {5, 7}};
+        for (int k = 0; k < 3; k++) {
+            double &a = nr[pairs[k][0] * P + c], &b = nr[pairs[k][1] * P + c];
+            const double v = 0.5 * (a + b);
+            a = v;
+            b = v;
+        }
+    }
+}
+
 // N_r re-embedded on another mesh: the displacements |d_a| < b_a between spins of a box of b
 // points, from index d mod m of the caller's mesh to d mod M of this one; the rest is zero (set
 // before).
@@ -974,6 +991,13 @@ cudaError_t build_nk_tiles(asd_handle* h, const double2* z, uint32_t ncomp, bool
         nk_tile_cplx<<<nbk(9 * Pk, 256), 256, 0, h->stream>>>(Pk, L.mesh[0], L.mesh[1], Kz, PT, z, scale, t);
         L.nkt = t;
     }
+    return cudaGetLastError();
+}
+
+cudaError_t prepare_nr(asd_handle* h, const uint32_t mesh[3], uint32_t clear, bool sym, double* d_nr) {
+    const uint3 m = make_uint3(mesh[0], mesh[1], mesh[2]);
+    const size_t P = (size_t)m.x * m.y * m.z;
+    prepare_nr_k<<<nbk(P, 256), 256, 0, h->stream>>>(m, clear, sym ? 1 : 0, d_nr);
     return cudaGetLastError();
 }
 

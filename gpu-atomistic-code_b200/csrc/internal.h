@@ -299,6 +299,9 @@ cudaError_t run_zy_part3(const LongRange& L, bool inverse, cudaStream_t st, bool
 cudaError_t build_plane_twiddles(asd_handle* h);
 bool plane_path_fits(const LongRange& L, bool cplx);
 void plane_mesh_for(const uint32_t box[3], uint32_t mesh[3]);
+// The caller's N_r on the device: the m/2 planes of the axes in `clear` zeroed, and the (a,b), (b,a)
+// pairs of a symmetric matrix replaced by their mean.
+cudaError_t prepare_nr(asd_handle* h, const uint32_t mesh[3], uint32_t clear, bool sym, double* d_nr);
 cudaError_t embed_nr(asd_handle* h, const uint32_t box[3], const uint32_t from[3], const uint32_t to[3],
                      const double* d_in, double* d_out);
 size_t plane_spectrum_elems(const LongRange& L);
