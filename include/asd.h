@@ -78,7 +78,8 @@ extern "C" {
                                                    the wait before a block retires keeps its bound;
                                                    asd_sync reports ASD_ETIMEOUT */
 #define ASD_FLAG_SERIAL_LAUNCH       (1u << 21) /* fused forms: launch the step kernels strictly one
-                                                   after another (no programmatic dependent launch:
+                                                   after another (no programmatic dependent launch,
+                                                   and no launch of several steps of a small lattice:
                                                    a comparison aid) */
 
 #define ASD_ALL_REPLICAS 0xFFFFFFFFu
@@ -313,7 +314,8 @@ int asd_kernel_table(const asd_handle* h, char* out, size_t out_len);
  * the typed exchange words), with ASD_FLAG_AUTOTUNE the autotuner's timings, and the transform
  * path of the long-range field. */
 int asd_tuning(const asd_handle* h, char* out, size_t out_len);
-/* Set the fused stage kernel's launch shape by hand: block in {64, 128, 256}; staging 1 stages
+/* Set the fused stage kernel's launch shape by hand (by default a matrix whose rows repeat runs by
+ * row patterns, which no staging mode selects): block in {64, 128, 256}; staging 1 stages
  * each block's typed exchange words in shared memory by bulk copy, staging 2 also the spans of
  * neighbour spins its rows read (each falls back to the lower mode where the layout is not
  * typed SELL or the data do not fit).  Results do not depend on the shape. */
