@@ -1250,7 +1250,10 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
         h->d_err = dalloc<uint32_t>(1);
         h->d_gridbar = dalloc<unsigned long long>(1);
         h->sell.err = h->d_err;
-        CK(cudaHostAlloc(reinterpret_cast<void**>(&h->h_err), sizeof(uint32_t), cudaHostAllocDefault));
+        CK(cudaHostAlloc(reinterpret_cast<void**>(&h->h_err), 2 * sizeof(uint32_t), cudaHostAllocDefault));
+        h->h_lost = h->h_err + 1;
+        *h->h_lost = 0;
+        CK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&h->d_lost), h->h_err + 1, 0));
         if (!plain) {
             if (p.flags & ASD_FLAG_AUTOTUNE) autotune(h);
             else configure_stage(h, 256, (int)STAGE_PATTERN);
@@ -1288,6 +1291,20 @@ int asd_destroy(asd_handle* h) {
     return ASD_OK;
 }
 
+// A wait at the several-steps kernel's barrier that ran out leaves the spins in the middle of a step:
+// every call that steps, samples or returns something formed from them fails from then on (the kernel
+// has set the host word by the time the stream is waited for, so the check costs nothing) until
+// asd_set_spins or asd_set_state brings new ones.
+static void require_spins(const asd_handle* h) {
+    if (h->h_lost && *h->h_lost)
+        throw Fail{ASD_ETIMEOUT, "a block's wait at the barrier between two stages ran out; the spins are invalid until "
+                                 "they are set again"};
+}
+// New spins are in place and the stream is idle.
+static void spins_are_valid(asd_handle* h) {
+    if (h->h_lost) *h->h_lost = 0;
+}
+
 // Device staging buffer of 3N doubles for the spin / field transfers, allocated on first use
 // and kept (no allocation or device-wide synchronisation per call).
 static double* aos_buffer(asd_handle* h) {
@@ -1319,6 +1336,7 @@ int asd_set_spins(asd_handle* h, const double* s, size_t n_spins) {
         CK(e);
         CK(e2);
         h->lr_scattered = false;
+        spins_are_valid(h);
     } catch (const Fail& f) { return fail(h, f); }
     return ASD_OK;
 }
@@ -1331,7 +1349,7 @@ static int read_back(asd_handle* h, int what, double* out, size_t n_spins) {
         if (h->p.precision == ASD_FP64_PLAIN && what != 2) {
             CK(cudaMemcpyAsync(out, what == 0 ? h->p_s : h->p_det, bytes, cudaMemcpyDeviceToHost, h->stream));
             CK(cudaStreamSynchronize(h->stream));
-            return ASD_OK;
+            return ASD_OK;                       // (the plain form has no such barrier)
         }
         double* d = aos_buffer(h);
         if (what == 2) flush_applied(h);
@@ -1340,6 +1358,7 @@ static int read_back(asd_handle* h, int what, double* out, size_t n_spins) {
         cudaError_t e2 = cudaStreamSynchronize(h->stream);
         CK(e);
         CK(e2);
+        require_spins(h);
     } catch (const Fail& f) { return fail(h, f); }
     return ASD_OK;
 }
@@ -1355,6 +1374,7 @@ int asd_get_field(asd_handle* h, double* o, size_t n) {
 int asd_step(asd_handle* h, uint64_t nsteps) {
     if (!h) return ASD_EINVAL;
     try {
+        require_spins(h);
         CK(cudaSetDevice(h->device));
         run_steps(h, nsteps);
         CK(cudaGetLastError());
@@ -1434,6 +1454,7 @@ int asd_get_state(asd_handle* h, void* buf, size_t* len) {
         get(h->d_rep_sqrtT_f, h->nrep * sizeof(float));
         if (h->d_ttm) get(h->d_ttm, sizeof(TtmDev));
         CK(cudaStreamSynchronize(h->stream));
+        require_spins(h);
         *len = need;
     } catch (const Fail& f) { return fail(h, f); }
     return ASD_OK;
@@ -1482,6 +1503,7 @@ int asd_set_state(asd_handle* h, const void* buf, size_t len) {
                h->nrep * sizeof(double));
         for (uint32_t r = 0; r < h->nrep; r++) h->h_rep_T[r] = sq[r] * sq[r];
         h->lr_scattered = false;    // the long-range input is formed again from these spins
+        spins_are_valid(h);
     } catch (const Fail& f) { return fail(h, f); }
     return ASD_OK;
 }
@@ -1495,12 +1517,7 @@ int asd_sync(asd_handle* h) {
         if (h->d_err) CK(cudaMemcpyAsync(h->h_err, h->d_err, sizeof e, cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
         if (h->d_err) e = *h->h_err;
-        if (e & 4u) {
-            CK(cudaMemset(h->d_err, 0, sizeof(uint32_t)));
-            CK(cudaMemset(h->d_gridbar, 0, sizeof(unsigned long long)));
-            CK(cudaStreamSynchronize(nullptr));           // before h->stream, which does not wait for it
-            throw Fail{ASD_ETIMEOUT, "a block's wait at the barrier between two stages ran out; the spins are invalid"};
-        }
+        require_spins(h);
         if (e & 2u) {
             CK(cudaMemset(h->d_err, 0, sizeof(uint32_t)));
             throw Fail{ASD_ETIMEOUT, "a long-range transform block's bulk-copy wait ran out; the long-range field of "
@@ -1742,6 +1759,7 @@ int asd_set_site_field_pulse(asd_handle* h, double amp, double t0, double sigma)
 int asd_sample_magnetisation(asd_handle* h) {
     if (!h) return ASD_EINVAL;
     try {
+        require_spins(h);
         CK(cudaSetDevice(h->device));
         CK(launch_magnetisation(h));
         CK(launch_mag_push(h));
@@ -1757,6 +1775,7 @@ int asd_magnetisation_stats(asd_handle* h, double* out, size_t out_len) {
         CK(cudaSetDevice(h->device));
         CK(cudaMemcpyAsync(out, h->d_stats, m * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
+        require_spins(h);
         for (size_t q = 0; q < m; q += 4) {           // M2 -> variance (n-1 normalised), inc/util.h:68-71
             const double n = out[q];
             out[q + 2] = n > 1 ? out[q + 2] / (n - 1) : 0.0;
@@ -1814,6 +1833,7 @@ int asd_sq_sample(asd_handle* h) {
     try {
         if (!h->sq.on) throw Fail{ASD_ESTATE, "asd_sq_setup has not been called"};
         if (h->sq.nsamples >= h->sq.max_samples) throw Fail{ASD_ESTATE, "S(q,t) series is full"};
+        require_spins(h);
         CK(cudaSetDevice(h->device));
         CK(launch_sq_sample(h));
     } catch (const Fail& f) { return fail(h, f); }
@@ -1829,6 +1849,7 @@ int asd_sq_get(asd_handle* h, double* out, size_t out_len, uint32_t* nsamples) {
         CK(cudaSetDevice(h->device));
         CK(cudaMemcpyAsync(out, h->sq.series, m * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
+        require_spins(h);
         if (nsamples) *nsamples = h->sq.nsamples;
     } catch (const Fail& f) { return fail(h, f); }
     return ASD_OK;
@@ -1854,6 +1875,7 @@ int asd_sq_spectrum(asd_handle* h, uint32_t window, double alpha, double beta, d
         d = dalloc<double>(2 * m);
         dp = dalloc<uint32_t>(2 * (size_t)nk);
         CK(launch_sq_spectrum(h, (int)window, alpha, beta, (uint32_t)pw, sample_dt, fcut_lo, fcut_hi, d, d + m, dp));
+        require_spins(h);
         if (raw) CK(cudaMemcpy(raw, d, m * sizeof(double), cudaMemcpyDeviceToHost));
         if (smooth) CK(cudaMemcpy(smooth, d + m, m * sizeof(double), cudaMemcpyDeviceToHost));
         if (peak_raw) CK(cudaMemcpy(peak_raw, dp, nk * sizeof(uint32_t), cudaMemcpyDeviceToHost));
@@ -1896,6 +1918,7 @@ int asd_magnetisation(asd_handle* h, double* out, size_t out_len) {
         if (!hout)
             CK(cudaMemcpyAsync(out, h->d_mag, (size_t)h->nrep * h->nsub * 3 * 8, cudaMemcpyDeviceToHost, h->stream));
         CK(cudaStreamSynchronize(h->stream));
+        require_spins(h);
     } catch (const Fail& f) { return fail(h, f); }
     return ASD_OK;
 }
@@ -1918,6 +1941,7 @@ int asd_time_steps(asd_handle* h, uint64_t nsteps, double* ms, uint64_t* launche
         CK(cudaEventSynchronize(h->kev[1]));
         float f = 0.f;
         CK(cudaEventElapsedTime(&f, h->kev[0], h->kev[1]));
+        require_spins(h);
         *ms = f;
         if (launches) *launches = h->launches - l0;
     } catch (const Fail& f) { return fail(h, f); }

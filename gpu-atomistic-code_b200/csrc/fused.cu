@@ -494,7 +494,6 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
 // with neighbours through L1), and a barrier over the grid (a counter in L2, waits bounded) stands
 // between the stages.
 constexpr uint32_t MAX_STAGES = 6;
-constexpr uint32_t ERR_RESIDENT_TIMEOUT = 4u;
 constexpr uint32_t RESIDENT_WAIT_POLLS = 1u << 21;     // about a second
 
 template <typename R>
@@ -502,13 +501,16 @@ struct ResidentArgs {
     StageArgs<R> st[MAX_STAGES];
     uint32_t nst;                // stages per step (2: Heun)
     uint32_t nsteps;
-    unsigned long long* barrier; // arrivals so far: a multiple of the grid between launches
-    uint32_t* err;
+    unsigned long long* barrier; // arrivals so far: 0 before a launch (advance_k), or a multiple of the grid
+    uint32_t* lost;              // page-locked host word: nonzero from a wait that ran out until new spins come
+    uint32_t give_up;            // ASD_FLAG_WAIT_TIMEOUT: a launch from step 0 gives up at its first wait
 };
 
 // The barrier in two halves: every block arrives once its stores are done, and waits until all have
 // (their stores are then visible); false when the wait ran out.  In between goes what does not
-// depend on the other blocks.
+// depend on the other blocks.  A block that gives up leaves the grid in the middle of a step, and the
+// others run out of their own waits: the host word tells the calls that read results, and advance_k
+// sets the arrivals back for the launches already queued, which step on from whatever it left.
 __device__ __forceinline__ void barrier_arrive(unsigned long long* arrivals, unsigned long long& target) {
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -518,16 +520,18 @@ __device__ __forceinline__ void barrier_arrive(unsigned long long* arrivals, uns
         else target += gridDim.x;
     }
 }
-__device__ __forceinline__ bool barrier_wait(unsigned long long* arrivals, unsigned long long target, uint32_t* err) {
+template <typename R>
+__device__ __forceinline__ bool barrier_wait(const ResidentArgs<R>& ra, unsigned long long target, uint32_t polls) {
     __shared__ uint32_t ok;
     if (threadIdx.x == 0) {
         unsigned long long v = 0;
         uint32_t it = 0;
-        do asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(arrivals) : "memory");
-        while (v < target && ++it < RESIDENT_WAIT_POLLS);
+        do asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(ra.barrier) : "memory");
+        while (v < target && ++it < polls);
         asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        ok = v >= target;
-        if (v < target) atomicOr(err, ERR_RESIDENT_TIMEOUT);
+        const bool all = v >= target && polls;
+        ok = all;
+        if (!all) *static_cast<volatile uint32_t*>(ra.lost) = 1u;
     }
     __syncthreads();
     return ok != 0;
@@ -543,6 +547,7 @@ __global__ void __launch_bounds__(256, 2)
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const bool row = i < c.n;
     const uint64_t t0 = *c.step_base;
+    const uint32_t polls = ra.give_up && t0 == 0 ? 0u : RESIDENT_WAIT_POLLS;
     uint32_t rep = 0;
     bool hot = false;
     x.lrn[0] = x.lrn[1] = x.lrn[2] = R(0);
@@ -571,13 +576,15 @@ __global__ void __launch_bounds__(256, 2)
             if (last && s + 1 == ra.nsteps) return;
             barrier_arrive(ra.barrier, target);
             if (last && hot) draw_thermal<R>(c, c.mat[atom_of(c, i)], rep, i, t0 + s + 1, x.lrn);
-            if (!barrier_wait(ra.barrier, target, ra.err)) return;
+            if (!barrier_wait(ra, target, polls)) return;
         }
 }
 
-__global__ void advance_k(uint64_t* step, uint32_t n) {
+// (and the several-steps kernel's arrivals back to zero: a launch whose wait ran out leaves any number)
+__global__ void advance_k(uint64_t* step, uint32_t n, unsigned long long* arrivals) {
     pdl_enter();
     *step += n;
+    *arrivals = 0;
 }
 // The det field is written at the step the device counter holds (the one-step graph's step).
 // The applied field rides in the parameters of this first node of the one-step graph: a new
@@ -784,7 +791,8 @@ ResidentArgs<float> resident_args(asd_handle* h, bool comp) {
         else for (int b = 0; b < 6; b++) a.k[b] = v3<float>(h->kf[b]);
     }
     ra.barrier = h->d_gridbar;
-    ra.err = h->d_err;
+    ra.lost = h->d_lost;
+    ra.give_up = (h->p.flags & ASD_FLAG_WAIT_TIMEOUT) ? 1u : 0u;
     return ra;
 }
 
@@ -927,8 +935,7 @@ cudaError_t launch_fused_step(asd_handle* h, uint32_t rel, bool) {
 // lattice is small, its matrix has patterns and nothing else runs between the stages; else step by step.
 cudaError_t launch_fused_steps(asd_handle* h, uint32_t k) {
     const bool one = k > 1 && h->n <= (h->full ? RESIDENT_MAX_FULL : RESIDENT_MAX) && h->p.precision == ASD_FP32 && h->dexch == ASD_EXCH_CSR &&
-                     h->sell.stage == STAGE_PATTERN && h->lr.mode == ASD_LR_NONE && !h->d_ttm && !h->sc.q4_ptr && step_pdl(h) &&
-                     !(h->p.flags & ASD_FLAG_WAIT_TIMEOUT);
+                     h->sell.stage == STAGE_PATTERN && h->lr.mode == ASD_LR_NONE && !h->d_ttm && !h->sc.q4_ptr && step_pdl(h);
     if (one) {
         const bool comp = (h->p.flags & ASD_FLAG_COMPENSATED) != 0, heun = h->p.integrator == ASD_HEUN;
         ResidentArgs<float> ra = resident_args(h, comp);
@@ -973,7 +980,8 @@ cudaError_t update_det_applied(asd_handle* h) {
 }
 
 cudaError_t launch_step_advance(asd_handle* h, uint32_t nsteps) {
-    const cudaError_t e = launch_step_kernel(advance_k, dim3(1), dim3(1), 0, h->stream, 1, step_pdl(h), h->d_step, nsteps);
+    const cudaError_t e = launch_step_kernel(advance_k, dim3(1), dim3(1), 0, h->stream, 1, step_pdl(h), h->d_step, nsteps,
+                                             h->d_gridbar);
     h->launches += 1;
     return e != cudaSuccess ? e : cudaGetLastError();
 }

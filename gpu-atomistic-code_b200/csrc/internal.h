@@ -213,7 +213,9 @@ struct asd_handle {
     std::vector<uint32_t> h_words;       // typed SELL words (host copy, for the local words)
     uint32_t* d_err = nullptr;           // device error bits (waits that ran out)
     unsigned long long* d_gridbar = nullptr; // arrivals at the grid barrier of the several-steps kernel
-    uint32_t* h_err = nullptr;           // page-locked host word the error bits are read into
+    uint32_t* h_err = nullptr;           // page-locked host words: the error bits as read back, and h_lost
+    volatile uint32_t* h_lost = nullptr; // set by the several-steps kernel when a wait at its barrier ran out
+    uint32_t* d_lost = nullptr;          // its device address
     double* d_aos = nullptr;             // [3N] staging buffer of the spin / field transfers
     unsigned long long* d_check = nullptr; // [2] first non-finite component, first zero-length spin
     uint32_t* d_rep_of_tile = nullptr;   // replica of each 32-spin tile's first spin

@@ -76,7 +76,9 @@ extern "C" {
                                                    kernels then read global memory, results unchanged;
                                                    the x transform leaves its tile, an invalid field);
                                                    the wait before a block retires keeps its bound;
-                                                   asd_sync reports ASD_ETIMEOUT */
+                                                   asd_sync reports ASD_ETIMEOUT.  A launch of several
+                                                   steps of a small lattice that starts from step 0
+                                                   gives up at its barrier as well (asd_step) */
 #define ASD_FLAG_SERIAL_LAUNCH       (1u << 21) /* fused forms: launch the step kernels strictly one
                                                    after another (no programmatic dependent launch,
                                                    and no launch of several steps of a small lattice:
@@ -158,7 +160,13 @@ int asd_get_det_field(asd_handle* h, double* hout, size_t n_spins);
  * (CH after the stage-1 field kernels, src/cufields.cu:201-203, 405). */
 int asd_get_field(asd_handle* h, double* hout, size_t n_spins);
 
-/* llg::integrate(t) x nsteps (src/llg.cpp:639-664 -> cullg::llgGPU / llgGPURK4 / llgGPURK5). */
+/* llg::integrate(t) x nsteps (src/llg.cpp:639-664 -> cullg::llgGPU / llgGPURK4 / llgGPURK5).
+ * Enqueues the steps and returns.  A small lattice runs several steps in one launch, whose blocks wait
+ * for one another between the stages; each wait is bounded (about a second).  Should one run out, the
+ * spins are left in the middle of a step: every call that steps, samples, or returns spins, fields,
+ * magnetisation, statistics, S(q,t) or state then fails with ASD_ETIMEOUT, as asd_sync does, until
+ * asd_set_spins or asd_set_state brings new spins (the step counter has moved on meanwhile, and
+ * statistics and series may hold samples of the invalid spins). */
 int asd_step(asd_handle* h, uint64_t nsteps);
 int asd_get_step(const asd_handle* h, uint64_t* t);
 int asd_set_step(asd_handle* h, uint64_t t);

@@ -4,7 +4,9 @@ block of the stage kernel reads its exchange words and neighbour spins from glob
 of shared memory, so the spins still match the oracle, and waits again (bounded) before retiring
 so no copy lands in a retired block; a timed-out block of the x transform leaves its tile and the
 long-range field of that evaluation is flagged invalid.  Either way asd_sync reports
-ASD_ETIMEOUT once and clears it, and the handle and the context stay usable."""
+ASD_ETIMEOUT once and clears it, and the handle and the context stay usable.  A block that gives up at
+the several-steps kernel's barrier leaves the spins invalid, which every call reports until new ones
+are set."""
 import numpy as np
 import pytest
 
@@ -57,3 +59,43 @@ def test_transform_wait_times_out_and_context_stays_usable(gpu):
         h.sync()
         g = h.get_spins()
     assert maxdiff(g, o.spins()) <= 1e-5, maxdiff(g, o.spins())
+
+
+@pytest.mark.parametrize("recover", ["set_spins", "set_state"])
+def test_several_steps_barrier_times_out_and_handle_recovers(gpu, recover):
+    """The grid barrier of the several-steps launch: when its wait runs out (the test aid: in a launch
+    from step 0) every call that returns or uses the spins says so, launches already queued return
+    at once, and new spins make the handle step as before: bit-identical to a handle that never
+    timed out, through whole chunks, a remainder and single steps."""
+    s = LT.sc_ferromagnet((20, 13, 11), T=80.0)          # 45 blocks
+    S0 = LT.random_spins(s.nspins, 2)
+    with A.Handle(A.RunParams(precision=A.FP32, flags=A.FLAG_COMPENSATED, seed=3), s) as h:
+        h.set_step(500)
+        h.set_spins(S0)
+        state = h.get_state()
+        h.step(70)
+        h.step(1)
+        want, mag = h.get_spins(), h.magnetisation()
+    with A.Handle(A.RunParams(precision=A.FP32, flags=A.FLAG_COMPENSATED | A.FLAG_WAIT_TIMEOUT, seed=3), s) as h:
+        h.set_spins(S0)
+        try:
+            for _ in range(4):
+                h.step(64)                               # queued behind the launch that gives up, or refused
+        except A.AsdError as ex:
+            assert ex.code == A.ASD_ETIMEOUT
+        for call in (h.get_spins, h.sync, h.magnetisation, h.get_field, h.get_det_field, h.get_state, h.sync,
+                     h.magnetisation_stats, h.sample_magnetisation, lambda: h.step(1), lambda: h.step(40)):
+            with pytest.raises(A.AsdError) as ex:
+                call()
+            assert ex.value.code == A.ASD_ETIMEOUT
+            assert "barrier" in str(ex.value)
+        if recover == "set_spins":
+            h.set_step(500)
+            h.set_spins(S0)
+        else:
+            h.set_state(state)
+        h.step(70)
+        h.step(1)
+        h.sync()
+        assert np.array_equal(h.get_spins(), want)
+        assert np.array_equal(h.magnetisation(), mag)
