@@ -53,6 +53,10 @@ T* dupload(const T* src, size_t n) {
     return p;
 }
 
+// dalloc's zeroing and the uploads run on the default stream, which the handles' non-blocking streams do
+// not wait for: called before work on h->stream touches what they filled.
+void uploads_done() { CK(cudaStreamSynchronize(nullptr)); }
+
 int fail(asd_handle* h, const Fail& f) {
     if (h) h->err = f.msg;
     return f.code;
@@ -525,8 +529,8 @@ void setup_lr(asd_handle* h, const asd_system& s, bool plain) {
     }
     const size_t P_in = (size_t)s.mesh[0] * s.mesh[1] * s.mesh[2];
     double* d_nr = dupload(s.nr, 9 * P_in);
+    uploads_done();
     if (!plain) {
-        CK(cudaStreamSynchronize(nullptr));                // the upload, which h->stream does not wait for
         const cudaError_t ep = prepare_nr(h, s.mesh, clear, sym, d_nr);
         if (ep != cudaSuccess) {
             cudaFree(d_nr);
@@ -665,6 +669,7 @@ bool build_spin_stage(asd_handle* h, int B) {
     }
     m.span_ptr = dupload(ptr.data(), ptr.size());
     m.spans = reinterpret_cast<uint4*>(dupload(spans.data(), spans.size()));
+    uploads_done();
     m.spin_slots = slots;
     m.spin_block = (uint32_t)B;
     return true;
@@ -1239,6 +1244,7 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
             h->d_sub_of_atom = dupload(h->h_sub_of_mat.data(), h->h_sub_of_mat.size());
         }
         // ---- default spins +z, then a graph for the fused forms
+        uploads_done();
         {
             std::vector<double> s3(3 * (size_t)n, 0.0);
             for (uint32_t i = 0; i < n; i++) s3[3 * (size_t)i + 2] = 1.0;
@@ -1249,6 +1255,7 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
         CK(cudaEventCreate(&h->kev[1]));
         h->d_err = dalloc<uint32_t>(1);
         h->d_gridbar = dalloc<unsigned long long>(1);
+        uploads_done();
         h->sell.err = h->d_err;
         CK(cudaHostAlloc(reinterpret_cast<void**>(&h->h_err), 2 * sizeof(uint32_t), cudaHostAllocDefault));
         h->h_lost = h->h_err + 1;
@@ -1269,7 +1276,6 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
             if (G > 4096) G = upd;
             build_graph(h, G);
         }
-        CK(cudaStreamSynchronize(nullptr));               // the zeroing of the buffers above
         CK(cudaStreamSynchronize(h->stream));
     } catch (const Fail& f) {
         g_create_err = f.msg;
@@ -1308,7 +1314,10 @@ static void spins_are_valid(asd_handle* h) {
 // Device staging buffer of 3N doubles for the spin / field transfers, allocated on first use
 // and kept (no allocation or device-wide synchronisation per call).
 static double* aos_buffer(asd_handle* h) {
-    if (!h->d_aos) h->d_aos = dalloc<double>(3 * (size_t)h->n);
+    if (!h->d_aos) {
+        h->d_aos = dalloc<double>(3 * (size_t)h->n);
+        uploads_done();
+    }
     return h->d_aos;
 }
 
@@ -1321,7 +1330,10 @@ int asd_set_spins(asd_handle* h, const double* s, size_t n_spins) {
         REQUIRE(s && n_spins == h->n, "spin array must hold 3*nspins doubles");
         CK(cudaSetDevice(h->device));
         double* d = aos_buffer(h);
-        if (!h->d_check) h->d_check = dalloc<unsigned long long>(2);
+        if (!h->d_check) {
+            h->d_check = dalloc<unsigned long long>(2);
+            uploads_done();
+        }
         unsigned long long bad[2] = {0, 0};
         cudaError_t e = cudaMemcpyAsync(d, s, 3 * n_spins * sizeof(double), cudaMemcpyHostToDevice, h->stream);
         if (e == cudaSuccess) e = launch_check_spins(h, d, h->d_check);
@@ -1519,12 +1531,12 @@ int asd_sync(asd_handle* h) {
         if (h->d_err) e = *h->h_err;
         require_spins(h);
         if (e & 2u) {
-            CK(cudaMemset(h->d_err, 0, sizeof(uint32_t)));
+            CK(cudaMemsetAsync(h->d_err, 0, sizeof(uint32_t), h->stream));
             throw Fail{ASD_ETIMEOUT, "a long-range transform block's bulk-copy wait ran out; the long-range field of "
                                      "that evaluation is invalid"};
         }
         if (e & 1u) {
-            CK(cudaMemset(h->d_err, 0, sizeof(uint32_t)));
+            CK(cudaMemsetAsync(h->d_err, 0, sizeof(uint32_t), h->stream));
             throw Fail{ASD_ETIMEOUT, "a stage kernel's shared-memory staging wait ran out; those blocks read the "
                                      "exchange words from global memory instead (results unaffected)"};
         }
@@ -1590,6 +1602,7 @@ int asd_set_four_spin(asd_handle* h, const uint32_t* xadj_jkl, const uint32_t* a
             }
             h->d_q4ptr = dupload(xadj_jkl, (size_t)h->n + 1);
             h->d_q4jkl = dupload(q.data(), q.size());
+            uploads_done();
             h->sc.q4_ptr = h->d_q4ptr;
             h->sc.q4_jkl = h->d_q4jkl;
             h->sc.q4_jq = JQ;
@@ -1623,6 +1636,7 @@ int asd_set_ttm(asd_handle* h, const asd_ttm* m) {
             for (uint32_t q = 0; q < m->npulses; q++) { d.scale[q] = m->pulse_scale[q]; d.delay[q] = m->pulse_delay[q]; }
             if (!h->d_ttm) CK(cudaMalloc(&h->d_ttm, sizeof(TtmDev)));
             CK(cudaMemcpy(h->d_ttm, &d, sizeof d, cudaMemcpyHostToDevice));
+            uploads_done();
             for (auto& T : h->h_rep_T) T = m->initial_T;   // the bath is hot from now on
         }
         if (h->graph_steps) build_graph(h, h->graph_steps);   // the step kernels change
@@ -1716,6 +1730,7 @@ int asd_set_site_field(asd_handle* h, const double* prof, size_t n_spins) {
             }
             if (!had) build_graph(h, h->graph_steps ? h->graph_steps : 32);  // kernels now read the profile
         }
+        uploads_done();
         // CsetStagFields resets the ramp: CHstg = CInitHstg
         set_dyn(h, DYN_STAG_SCALE, 1.0);
         h->stag_rv = 1.0;
@@ -1820,6 +1835,7 @@ int asd_sq_setup(asd_handle* h, uint32_t qaxis, const double* uo, const uint32_t
         S.kidx = dupload(kidx.data(), kidx.size());
         S.grid = dalloc<double2>(P);
         S.series = dalloc<double2>((size_t)max_samples * nk);
+        uploads_done();
         int dims[3] = {(int)mesh[0], (int)mesh[1], (int)mesh[2]};
         CKFFT(cufftPlanMany(&S.plan, 3, dims, nullptr, 1, (int)P, nullptr, 1, (int)P, CUFFT_Z2Z, 1));
         CKFFT(cufftSetStream(S.plan, h->stream));
@@ -1874,6 +1890,7 @@ int asd_sq_spectrum(asd_handle* h, uint32_t window, double alpha, double beta, d
         CK(cudaSetDevice(h->device));
         d = dalloc<double>(2 * m);
         dp = dalloc<uint32_t>(2 * (size_t)nk);
+        uploads_done();
         CK(launch_sq_spectrum(h, (int)window, alpha, beta, (uint32_t)pw, sample_dt, fcut_lo, fcut_hi, d, d + m, dp));
         require_spins(h);
         if (raw) CK(cudaMemcpy(raw, d, m * sizeof(double), cudaMemcpyDeviceToHost));
