@@ -151,95 +151,40 @@ __device__ __forceinline__ void draw_thermal(const StepConst& c, const MatConst&
     for (int q = 0; q < 3; q++) lrn[q] = xi[q] * tp;
 }
 
-// What a row needs beside the arguments: the block's staged words, spins and table, and the row's
-// pattern with its first words.
-template <typename R>
-struct RowCtx {
-    const uint32_t* staged = nullptr;
-    const uint16_t* staged16 = nullptr;
-    const R* sspin = nullptr;
-    uint32_t wbase = 0;
-    R* tab = nullptr;
-    uint64_t* bar = nullptr;
-    uint32_t pid = 0;
-    PatBatch<R, PAT_BATCH> first;
-    R lrn[3];                    // LIVE: the step's thermal field
-};
-
-// One stage of row i at step t.  K: the stage kind at compile time (1 Heun predictor, 2 Heun
-// corrector, 3 RK stage before the last, 4 last RK stage); a.kind still carries the RK stage
-// index.  LIVE: other blocks of the same launch write the spins it gathers.
-template <typename R, int EX, bool FULL, bool COMP, int K, bool LIVE>
-__device__ __forceinline__ void stage_row(const StepConst& c, const SellDev& sell, const PatDev& pat, const DiaDev& dia,
-                                          const StageArgs<R>& a, const uint32_t i, const uint64_t t, RowCtx<R>& x) {
-    constexpr bool EARLY = EX == EXCH_PATTERN_EARLY;
-    const bool early = EARLY && pat.W >= PAT_BATCH;
-    // stage spin at this site; the pattern kernels load it with the gather's first loads
-    R sv[3];
-    if constexpr (EARLY) {
-        for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
-        if (early) x.first.template spins<LIVE>(i, a.src);
-    }
-    const uint32_t at = atom_of(c, i);
-    const MatConst& mc = c.mat[at];
-    const uint32_t r = replica_of(c, i);
-    constexpr bool F32 = sizeof(R) == 4;
-    // one thermal draw per spin and step serves every stage (src/cuint.cu:72): the first stage
-    // draws it, later stages of the step load what the first stored
-    R lrn[3] = {R(0), R(0), R(0)};
-    if constexpr (LIVE) {
-        for (int q = 0; q < 3; q++) lrn[q] = x.lrn[q];    // drawn behind the barrier before the step
-    } else if (a.nz_mode == 2) {
-        if (is_hot<R>(c, r)) { lrn[0] = a.nz.p[0][i]; lrn[1] = a.nz.p[1][i]; lrn[2] = a.nz.p[2][i]; }
-    } else if (is_hot<R>(c, r)) {
-        draw_thermal<R>(c, mc, r, i, t, lrn);
-        if (a.nz_mode == 1) { a.nz.p[0][i] = lrn[0]; a.nz.p[1][i] = lrn[1]; a.nz.p[2][i] = lrn[2]; }
-    }
-    // the long-range field at this site: with diagonal tensors it is loaded before the staging
-    // wait, so that its two dependent loads (mesh index, field) overlap the copies and the
-    // gather; the full-tensor kernels have no registers to spare and load it after the gather
+// The long-range field at a site and its mesh point (two dependent loads).
+struct LrAt {
     uint32_t midx = 0;
-    float hl[3] = {0.f, 0.f, 0.f};
-    auto load_lr = [&]() {
-        if (a.lr.hr || a.lr.mr) midx = __ldg(a.lr.idx + i);
-        if (a.lr.hr) {
-            hl[0] = __ldg(a.lr.hr + midx);
-            hl[1] = __ldg(a.lr.hr + a.lr.P + midx);
-            hl[2] = __ldg(a.lr.hr + 2 * a.lr.P + midx);
-        }
-    };
-    if constexpr (!FULL) load_lr();
-    bool stage_timeout = false;
-    const uint32_t polls = (c.flags & ASD_FLAG_WAIT_TIMEOUT) ? 0u : STAGE_WAIT_POLLS;
-    if ((x.staged || x.staged16) && !mbar_wait_bounded(x.bar, polls)) {
-        // the copy did not land in time: record it and read the words and the table from
-        // global memory
-        atomicOr(sell.err, ERR_STAGE_TIMEOUT);
-        x.staged = nullptr;    // the global words carry global columns
-        x.staged16 = nullptr;
-        x.sspin = nullptr;
-        x.tab = const_cast<R*>(table_of<R>(sell));
-        stage_timeout = true;
+    float h[3] = {0.f, 0.f, 0.f};
+};
+template <typename R>
+__device__ __forceinline__ void load_lr(const StageArgs<R>& a, uint32_t i, LrAt& l) {
+    if (a.lr.hr || a.lr.mr) l.midx = __ldg(a.lr.idx + i);
+    if (a.lr.hr) {
+        l.h[0] = __ldg(a.lr.hr + l.midx);
+        l.h[1] = __ldg(a.lr.hr + a.lr.P + l.midx);
+        l.h[2] = __ldg(a.lr.hr + 2 * a.lr.P + l.midx);
     }
-    R h[3] = {R(0), R(0), R(0)};
-    if constexpr (is_pattern<EX> && !EARLY)
-        for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
-    if constexpr (EX == ASD_EXCH_CSR) gather_sell<R, FULL>(sell, i, a.src, x.tab, h, x.staged, x.wbase, x.sspin, x.staged16);
-    if constexpr (EX == ASD_EXCH_DIA) gather_dia<R, FULL>(dia, c.n, i, a.src, x.tab, h);
-    if constexpr (is_pattern<EX>) {
-        if (early) x.first.template add<FULL>(x.tab, h);
-        gather_pattern<R, FULL, LIVE>(pat, x.pid, i, a.src, x.tab, h, early ? PAT_BATCH : 0u);
-    }
+}
+
+// The stage kernels' common part behind the exchange gather, in two functions.  (The front, to the end
+// of the gather, stands in the kernels themselves: as one function for all layouts it compiled to SELL
+// kernels 1.0 to 2.4 % slower at the same registers: sc 128³ of words 122.2 → 123.9 µs per step,
+// fcc-like 32³ 9.50 → 9.72; these two functions cost nothing.)
+// h += four-spin, long-range, site, thermal and applied fields.
+template <typename R, bool FULL>
+__device__ __forceinline__ void add_fields(const StepConst& c, const StageArgs<R>& a, const uint32_t i, const uint64_t t,
+                                           const R lrn[3], LrAt& l, R h[3]) {
+    constexpr bool F32 = sizeof(R) == 4;
     if (c.q4_ptr) {
         R h4[3];
         four_spin<R>(c, i, [&](uint32_t j, R v[3]) { v[0] = a.src.p[0][j]; v[1] = a.src.p[1][j]; v[2] = a.src.p[2][j]; }, h4);
         h[0] += h4[0]; h[1] += h4[1]; h[2] += h4[2];
     }
-    if constexpr (FULL) load_lr();
+    if constexpr (FULL) load_lr(a, i, l);
     if (a.lr.hr) {
-        h[0] += (R)(hl[0] * a.lr.inv_p);
-        h[1] += (R)(hl[1] * a.lr.inv_p);
-        h[2] += (R)(hl[2] * a.lr.inv_p);
+        h[0] += (R)(l.h[0] * a.lr.inv_p);
+        h[1] += (R)(l.h[1] * a.lr.inv_p);
+        h[2] += (R)(l.h[2] * a.lr.inv_p);
     }
     const double* dyn = c.dyn;
     const R* dynr;
@@ -252,9 +197,16 @@ __device__ __forceinline__ void stage_row(const StepConst& c, const SellDev& sel
     h[0] += lrn[0] + dynr[DYN_APPLIED];
     h[1] += lrn[1] + dynr[DYN_APPLIED + 1];
     h[2] += lrn[2] + dynr[DYN_APPLIED + 2];
+}
 
-    if constexpr (!is_pattern<EX>)
-        for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
+// Anisotropy, torque and update of row i with the stage spin sv and the total field h.  K: the stage
+// kind at compile time (1 Heun predictor, 2 Heun corrector, 3 RK stage before the last, 4 last RK
+// stage); a.kind still carries the RK stage index.
+template <typename R, bool COMP, int K>
+__device__ __forceinline__ void finish_row(const StepConst& c, const StageArgs<R>& a, const MatConst& mc, const uint32_t i,
+                                           const uint64_t t, const uint32_t midx, const R lrn[3], R h[3], R sv[3]) {
+    constexpr bool F32 = sizeof(R) == 4;
+    const double* dyn = c.dyn;
     const int kind = a.kind;
     if constexpr (K >= 3) {
         if (kind >= 11 && (c.flags & ASD_FLAG_RK_STAGE_SPIN_MIXED)) sv[1] = a.base.p[1][i];
@@ -348,24 +300,36 @@ __device__ __forceinline__ void stage_row(const StepConst& c, const SellDev& sel
         a.lr.mr[a.lr.P + midx] = (float)out[1] * wv;
         a.lr.mr[2 * a.lr.P + midx] = (float)out[2] * wv;
     }
-    // a block must not retire while its bulk copy may still be writing shared memory
-    if (stage_timeout) mbar_wait_bounded(x.bar, STAGE_WAIT_POLLS);
+}
+
+// The block's rows of every per-spin input: one bulk L2 prefetch each, so the loads after the exchange
+// gather find them in L2; sizes stop at the last row (whole 16-byte units), so no prefetch reaches
+// past an array.
+template <typename R>
+__device__ __forceinline__ void prefetch_rows(const StepConst& c, const StageArgs<R>& a) {
+    const uint32_t r0 = blockIdx.x * blockDim.x;
+    const uint32_t rows = min(blockDim.x, c.n - r0);
+    const uint32_t bytes = (rows * (uint32_t)sizeof(R)) & ~15u;
+    if (bytes)
+        for (uint32_t q = 0; q < a.npf; q++)
+            bulk_prefetch_l2(static_cast<const char*>(a.pf[q]) + (size_t)r0 * sizeof(R), bytes);
 }
 
 template <typename R, int EX, bool FULL, bool COMP, int K>
 __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
-    stage_kernel(const StepConst c, const SellDev sell, const PatDev pat, const DiaDev dia, const StageArgs<R> a) {
+    stage_kernel(const StepConst c, const SellDev sell, const DiaDev dia, const StageArgs<R> a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t stage_bar;
     R* tab = reinterpret_cast<R*>(smem_raw);
     // Until pdl_enter below the block touches only set-up data (the exchange words, the tensor
     // table, the spans, the mesh index): the copies of the words and the table start while the
     // previous kernel's last blocks run; the neighbour-spin spans are copied after the wait.
-    RowCtx<R> x;
-    x.bar = &stage_bar;
+    const uint32_t* staged = nullptr;
+    const uint16_t* staged16 = nullptr;
+    const R* sspin = nullptr;
     R* span_dst = nullptr;           // shared-memory spin buffer the span copies fill after the wait
     uint32_t span0 = 0, nspan = 0;
-    uint32_t& wbase = x.wbase;
+    uint32_t wbase = 0;
     if constexpr (EX == ASD_EXCH_CSR) {
         if (sell.typed) {
             // the tensor table: with staging, one more bulk copy on the staging barrier; else a
@@ -405,8 +369,8 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
                         if (threadIdx.x == 0) bulk_copy_stream(wbuf, sell.lwords16 + wbase, bytes16, &stage_bar);
                         if (threadIdx.x == 1) bulk_copy(tab, table_of<R>(sell), tab_bytes, &stage_bar);
                     }
-                    x.staged16 = wbuf;
-                    x.sspin = sbuf;
+                    staged16 = wbuf;
+                    sspin = sbuf;
                     span_dst = sbuf; span0 = sp0; nspan = nsp;
                     tab_staged = true;
                 } else if (!w16 && bytes) {
@@ -425,8 +389,8 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
                             bulk_copy_stream(wbuf, (nsp ? sell.lwords : sell.typed) + wbase, bytes, &stage_bar);
                         if (threadIdx.x == 1) bulk_copy(tab, table_of<R>(sell), tab_bytes, &stage_bar);
                     }
-                    x.staged = wbuf;
-                    if (nsp) { x.sspin = sbuf; span_dst = sbuf; span0 = sp0; nspan = nsp; }
+                    staged = wbuf;
+                    if (nsp) { sspin = sbuf; span_dst = sbuf; span0 = sp0; nspan = nsp; }
                     tab_staged = true;
                 }
             }
@@ -435,27 +399,6 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
     }
     if constexpr (EX == ASD_EXCH_DIA) {
         if (dia.dtype) load_table<R>(table_of<R>(dia), table_stride<FULL>() *dia.ntypes, tab);
-    }
-    // Row patterns (PatDev): no words to stage and no wait.  The stage reads 2 bytes of matrix per
-    // row instead of 28 (sc, 6 neighbours) or 108 (BCT-2, 26), and the pattern's entries come
-    // from L1, so all of the row's gathers are issued at once.  Measured against the fastest of the
-    // staged SELL shapes (step time in the graph, one B200): sc 128³ at 300 K 119.2 → 91.6 µs,
-    // 24 sc replicas (2.7 M spins) 155.0 → 121.6, sc 128×128×64 with dipole 175.9 → 163.0, BCT-2
-    // 64³ 55.4 → 49.2, sc 16³ 8.9 → 7.7.
-    // EARLY (FP32 lattices of at most one wave): the time of a stage is its chain of dependent loads,
-    // so the pattern's first words are read before the dependent-launch wait and their neighbours
-    // right after it, ahead of the thermal draw, and no L2 prefetch is issued (the state is in L2).
-    // µs per step: sc 16³ at 300 K 7.16 → 6.78, BCT-2 37×29×23 14.7 → 13.0; in FP64 (72 registers of
-    // neighbours held across the draw) it loses: 64×64×32 with dipole 45.7 → 47.6.
-    constexpr bool EARLY = EX == EXCH_PATTERN_EARLY;
-    const bool early = EARLY && pat.W >= PAT_BATCH;
-    if constexpr (is_pattern<EX>) {
-        const uint32_t row = blockIdx.x * blockDim.x + threadIdx.x;
-        if (row < c.n) x.pid = __ldg(pat.row + row);
-        if constexpr (EARLY)
-            if (early && row < c.n) x.first.words(reinterpret_cast<const int2*>(pat.ent + (size_t)x.pid * pat.W));
-        if constexpr (FULL) load_table<R>(table_of<R>(sell), table_stride<FULL>() * sell.ntypes, tab);
-        else tab = const_cast<R*>(table_of<R>(sell));
     }
     pdl_enter();
     if constexpr (EX == ASD_EXCH_CSR) {
@@ -468,21 +411,138 @@ __global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
                           &stage_bar);
             }
     }
-    if (!EARLY && threadIdx.x == 0 && a.npf) {
-        // the block's rows of every per-spin input: one bulk L2 prefetch each, so the loads
-        // after the exchange gather find them in L2; sizes stop at the last row (whole
-        // 16-byte units), so no prefetch reaches past an array
-        const uint32_t r0 = blockIdx.x * blockDim.x;
-        const uint32_t rows = min(blockDim.x, c.n - r0);
-        const uint32_t bytes = (rows * (uint32_t)sizeof(R)) & ~15u;
-        if (bytes)
-            for (uint32_t q = 0; q < a.npf; q++)
-                bulk_prefetch_l2(static_cast<const char*>(a.pf[q]) + (size_t)r0 * sizeof(R), bytes);
-    }
+    if (threadIdx.x == 0 && a.npf) prefetch_rows(c, a);
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.n) return;     // thread 0 of every block has i < n and always waits below
-    x.tab = tab;
-    stage_row<R, EX, FULL, COMP, K, false>(c, sell, pat, dia, a, i, *c.step_base + a.rel, x);
+    const uint64_t t = *c.step_base + a.rel;
+    const uint32_t at = atom_of(c, i);
+    const MatConst& mc = c.mat[at];
+    const uint32_t r = replica_of(c, i);
+    constexpr bool F32 = sizeof(R) == 4;
+    // one thermal draw per spin and step serves every stage (src/cuint.cu:72): the first stage
+    // draws it, later stages of the step load what the first stored
+    R lrn[3] = {R(0), R(0), R(0)};
+    bool hot;
+    if constexpr (F32) hot = __ldg(c.rep_sqrtT_f + r) > 0.0f; else hot = __ldg(c.rep_sqrtT + r) > 0.0;
+    if (hot && a.nz_mode == 2) {
+        lrn[0] = a.nz.p[0][i]; lrn[1] = a.nz.p[1][i]; lrn[2] = a.nz.p[2][i];
+    } else if (hot) {
+        if constexpr (F32) {
+            float xi[3];
+            thermal_normals_f(c.seed, __ldg(c.rep_stream + r), i - __ldg(c.rep_off + r), t, xi);
+            const float tp = __ldg(c.rep_sqrtT_f + r) * mc.sigma_f;
+            lrn[0] = xi[0] * tp; lrn[1] = xi[1] * tp; lrn[2] = xi[2] * tp;
+        } else {
+            double xi[3];
+            thermal_normals(c.seed, __ldg(c.rep_stream + r), i - __ldg(c.rep_off + r), t, xi);
+            const double tp = __ldg(c.rep_sqrtT + r) * mc.sigma;
+            lrn[0] = xi[0] * tp; lrn[1] = xi[1] * tp; lrn[2] = xi[2] * tp;
+        }
+        if (a.nz_mode == 1) { a.nz.p[0][i] = lrn[0]; a.nz.p[1][i] = lrn[1]; a.nz.p[2][i] = lrn[2]; }
+    }
+    // the long-range field at this site: with diagonal tensors it is loaded before the staging
+    // wait, so that its two dependent loads (mesh index, field) overlap the copies and the
+    // gather; the full-tensor kernels have no registers to spare and load it after the gather
+    LrAt l;
+    if constexpr (!FULL) load_lr(a, i, l);
+    bool stage_timeout = false;
+    const uint32_t polls = (c.flags & ASD_FLAG_WAIT_TIMEOUT) ? 0u : STAGE_WAIT_POLLS;
+    if ((staged || staged16) && !mbar_wait_bounded(&stage_bar, polls)) {
+        // the copy did not land in time: record it and read the words and the table from
+        // global memory
+        atomicOr(sell.err, ERR_STAGE_TIMEOUT);
+        staged = nullptr;      // the global words carry global columns
+        staged16 = nullptr;
+        sspin = nullptr;
+        tab = const_cast<R*>(table_of<R>(sell));
+        stage_timeout = true;
+    }
+    R h[3] = {R(0), R(0), R(0)};
+    if constexpr (EX == ASD_EXCH_CSR) gather_sell<R, FULL>(sell, i, a.src, tab, h, staged, wbase, sspin, staged16);
+    if constexpr (EX == ASD_EXCH_DIA) gather_dia<R, FULL>(dia, c.n, i, a.src, tab, h);
+    add_fields<R, FULL>(c, a, i, t, lrn, l, h);
+    R sv[3] = {a.src.p[0][i], a.src.p[1][i], a.src.p[2][i]};
+    finish_row<R, COMP, K>(c, a, mc, i, t, l.midx, lrn, h, sv);
+    // a block must not retire while its bulk copy may still be writing shared memory
+    if (stage_timeout) mbar_wait_bounded(&stage_bar, STAGE_WAIT_POLLS);
+}
+
+// ---- row patterns ----
+// What a row keeps beside the arguments: the tensor table, its pattern and the pattern's first words.
+template <typename R>
+struct RowCtx {
+    R* tab = nullptr;
+    uint32_t pid = 0;
+    PatBatch<R, PAT_BATCH> first;
+    R lrn[3];                    // LIVE: the step's thermal field
+};
+
+// One stage of row i at step t.  LIVE: other blocks of the same launch write the spins it gathers.
+template <typename R, int EX, bool FULL, bool COMP, int K, bool LIVE>
+__device__ __forceinline__ void pattern_row(const StepConst& c, const PatDev& pat, const StageArgs<R>& a, const uint32_t i,
+                                            const uint64_t t, RowCtx<R>& x) {
+    constexpr bool EARLY = EX == EXCH_PATTERN_EARLY;
+    const bool early = EARLY && pat.W >= PAT_BATCH;
+    // the stage spin at this site is loaded with the gather's first loads
+    R sv[3];
+    if constexpr (EARLY) {
+        for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
+        if (early) x.first.template spins<LIVE>(i, a.src);
+    }
+    const MatConst& mc = c.mat[atom_of(c, i)];
+    const uint32_t r = replica_of(c, i);
+    R lrn[3] = {R(0), R(0), R(0)};
+    if constexpr (LIVE) {
+        for (int q = 0; q < 3; q++) lrn[q] = x.lrn[q];    // drawn behind the barrier before the step
+    } else if (a.nz_mode == 2) {
+        if (is_hot<R>(c, r)) { lrn[0] = a.nz.p[0][i]; lrn[1] = a.nz.p[1][i]; lrn[2] = a.nz.p[2][i]; }
+    } else if (is_hot<R>(c, r)) {
+        draw_thermal<R>(c, mc, r, i, t, lrn);
+        if (a.nz_mode == 1) { a.nz.p[0][i] = lrn[0]; a.nz.p[1][i] = lrn[1]; a.nz.p[2][i] = lrn[2]; }
+    }
+    LrAt l;
+    if constexpr (!FULL) load_lr(a, i, l);
+    R h[3] = {R(0), R(0), R(0)};
+    if constexpr (!EARLY)
+        for (int q = 0; q < 3; q++) sv[q] = a.src.p[q][i];
+    if (early) x.first.template add<FULL>(x.tab, h);
+    gather_pattern<R, FULL, LIVE>(pat, x.pid, i, a.src, x.tab, h, early ? PAT_BATCH : 0u);
+    add_fields<R, FULL>(c, a, i, t, lrn, l, h);
+    finish_row<R, COMP, K>(c, a, mc, i, t, l.midx, lrn, h, sv);
+}
+
+// Row patterns (PatDev): no words to stage and no wait.  The stage reads 2 bytes of matrix per
+// row instead of 28 (sc, 6 neighbours) or 108 (BCT-2, 26), and the pattern's entries come
+// from L1, so all of the row's gathers are issued at once.  Measured against the fastest of the
+// staged SELL shapes (step time in the graph, one B200): sc 128³ at 300 K 119.2 → 91.6 µs,
+// 24 sc replicas (2.7 M spins) 155.0 → 121.6, sc 128×128×64 with dipole 175.9 → 163.0, BCT-2
+// 64³ 55.4 → 49.2, sc 16³ 8.9 → 7.7.
+// EARLY (FP32 lattices of at most one wave): the time of a stage is its chain of dependent loads,
+// so the pattern's first words are read before the dependent-launch wait and their neighbours
+// right after it, ahead of the thermal draw, and no L2 prefetch is issued (the state is in L2).
+// µs per step: sc 16³ at 300 K 7.16 → 6.78, BCT-2 37×29×23 14.7 → 13.0; in FP64 (36 registers of
+// neighbours held across the draw) it loses: 64×64×32 with dipole 45.7 → 47.6.
+template <typename R, int EX, bool FULL, bool COMP, int K>
+__global__ void __launch_bounds__(256, MinBlocks<R, EX, FULL, K>::value)
+    pattern_kernel(const StepConst c, const SellDev sell, const PatDev pat, const StageArgs<R> a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    constexpr bool EARLY = EX == EXCH_PATTERN_EARLY;
+    RowCtx<R> x;
+    // set-up data only before pdl_enter
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < c.n) x.pid = __ldg(pat.row + i);
+    if constexpr (EARLY)
+        if (pat.W >= PAT_BATCH && i < c.n) x.first.words(reinterpret_cast<const int2*>(pat.ent + (size_t)x.pid * pat.W));
+    if constexpr (FULL) {
+        x.tab = reinterpret_cast<R*>(smem_raw);
+        load_table<R>(table_of<R>(sell), table_stride<FULL>() * sell.ntypes, x.tab);
+    } else {
+        x.tab = const_cast<R*>(table_of<R>(sell));
+    }
+    pdl_enter();
+    if (!EARLY && threadIdx.x == 0 && a.npf) prefetch_rows(c, a);
+    if (i >= c.n) return;
+    pattern_row<R, EX, FULL, COMP, K, false>(c, pat, a, i, *c.step_base + a.rel, x);
 }
 
 // ---- several steps in one launch (small lattices) ----
@@ -558,7 +618,6 @@ __global__ void __launch_bounds__(256, 2)
         hot = is_hot<R>(c, rep);
         if (hot) draw_thermal<R>(c, c.mat[atom_of(c, i)], rep, i, t0, x.lrn);
     }
-    const DiaDev none{};
     unsigned long long target = 0;
     for (uint32_t s = 0; s < ra.nsteps; s++)
         for (uint32_t q = 0; q < ra.nst; q++) {
@@ -566,11 +625,11 @@ __global__ void __launch_bounds__(256, 2)
             if (row) {
                 constexpr int EX = EXCH_PATTERN_EARLY;
                 if constexpr (HEUN) {
-                    if (q == 0) stage_row<R, EX, FULL, COMP, 1, true>(c, sell, pat, none, ra.st[0], i, t0 + s, x);
-                    else stage_row<R, EX, FULL, COMP, 2, true>(c, sell, pat, none, ra.st[1], i, t0 + s, x);
+                    if (q == 0) pattern_row<R, EX, FULL, COMP, 1, true>(c, pat, ra.st[0], i, t0 + s, x);
+                    else pattern_row<R, EX, FULL, COMP, 2, true>(c, pat, ra.st[1], i, t0 + s, x);
                 } else {
-                    if (!last) stage_row<R, EX, FULL, COMP, 3, true>(c, sell, pat, none, ra.st[q], i, t0 + s, x);
-                    else stage_row<R, EX, FULL, COMP, 4, true>(c, sell, pat, none, ra.st[q], i, t0 + s, x);
+                    if (!last) pattern_row<R, EX, FULL, COMP, 3, true>(c, pat, ra.st[q], i, t0 + s, x);
+                    else pattern_row<R, EX, FULL, COMP, 4, true>(c, pat, ra.st[q], i, t0 + s, x);
                 }
             }
             if (last && s + 1 == ra.nsteps) return;
@@ -652,16 +711,16 @@ cudaError_t launch_stage_k(asd_handle* hd, const StageArgs<R>& a) {
     }
     if (is_pattern<EX> && FULL) smem = sizeof(R) * table_stride<FULL>() * hd->sell.ntypes;
     if (EX == ASD_EXCH_DIA && hd->dia.dtype) smem = sizeof(R) * table_stride<FULL>() *hd->dia.ntypes;
-    {
-        const cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(stage_kernel<R, EX, FULL, COMP, K>), smem);
+    auto launch = [&](auto kern, auto... args) {
+        cudaError_t e = raise_smem_limit(reinterpret_cast<const void*>(kern), smem);
         if (e != cudaSuccess) return e;
-    }
-    timer_begin(hd);
-    {
-        const cudaError_t e = launch_step_kernel(stage_kernel<R, EX, FULL, COMP, K>, dim3(grid), dim3(B), smem,
-                                                 hd->stream, 1, step_pdl(hd), hd->sc, hd->sell, hd->pat, hd->dia, a);
-        if (e != cudaSuccess) return e;
-    }
+        timer_begin(hd);
+        return launch_step_kernel(kern, dim3(grid), dim3(B), smem, hd->stream, 1, step_pdl(hd), hd->sc, hd->sell, args..., a);
+    };
+    cudaError_t e;
+    if constexpr (is_pattern<EX>) e = launch(pattern_kernel<R, EX, FULL, COMP, K>, hd->pat);
+    else e = launch(stage_kernel<R, EX, FULL, COMP, K>, hd->dia);
+    if (e != cudaSuccess) return e;
     hd->launches += 1;
     if (hd->timing) {
         const bool typed = (EX == ASD_EXCH_CSR && hd->sell.typed) || is_pattern<EX> || (EX == ASD_EXCH_DIA && hd->dia.dtype);
