@@ -163,6 +163,9 @@ void build_patterns(asd_handle* h, const std::vector<uint32_t>& xadj, const std:
     std::unordered_multimap<uint64_t, uint32_t> seen;  // hash of a pattern -> its number
     std::vector<int32_t> cur(W);
     const size_t most = std::min<size_t>(65536, adj.size() / (4 * (size_t)W));
+    constexpr uint32_t WINDOW = 1024;                  // rows an SM holds at a time
+    std::vector<uint32_t> last;                        // window in which a pattern last came, plus one
+    uint64_t fresh = 0;                                // patterns met for the first time in a window
     auto word = [](uint32_t col, uint32_t i, uint32_t typ) { return (int32_t)(((col - i) << 8) | typ); };
     for (uint32_t i = 0; i < n; i++) {
         const uint32_t len = xadj[i + 1] - xadj[i];
@@ -192,11 +195,16 @@ void build_patterns(asd_handle* h, const std::vector<uint32_t>& xadj, const std:
                 if (p >= most) return;
                 ent.insert(ent.end(), cur.begin(), cur.end());
                 plen.push_back(len);
+                last.push_back(0);
                 seen.emplace(hash, p);
             }
         }
         row[i] = (uint16_t)p;
+        if (last[p] != i / WINDOW + 1) { last[p] = i / WINDOW + 1; fresh++; }
     }
+    // words of the patterns a window reads, per row: below one, the words themselves (W per row) cost more
+    // whatever the lattice; above, the scattered reads decide
+    h->pat_varied = (double)fresh * W > (double)n;
     h->pat.W = W;
     h->pat.npat = (uint32_t)plen.size();
     h->pat.row = dupload(row.data(), row.size());
@@ -697,6 +705,52 @@ void configure_stage(asd_handle* h, int B, int mode) {
         if (h->sell.spin_block != (uint32_t)B && !build_spin_stage(h, B)) return;
         if (h->sell.spin_block == (uint32_t)B) h->sell.stage = 2;
     }
+}
+
+// All spins along +z.
+void set_default_spins(asd_handle* h) {
+    std::vector<double> s3(3 * (size_t)h->n, 0.0);
+    for (uint32_t i = 0; i < h->n; i++) s3[3 * (size_t)i + 2] = 1.0;
+    const int rc = asd_set_spins(h, s3.data(), h->n);
+    if (rc != ASD_OK) throw Fail{rc, h->err};
+}
+
+// A matrix of many patterns (an alloy whose pair tensors go with the species: 2 to the power of W + 1
+// neighbourhoods) reads its pattern words scattered, where the SELL words are coalesced: neither is the
+// better one by a rule on sizes.  FP32 alloys of 2 species, step time of the patterns as a multiple of the
+// words': diagonal tensors, 12 neighbours 0.73 (52³) to 1.09 (56³), 14 neighbours 0.71 to 1.08; full
+// tensors 0.75 to 1.30 and 0.75 to 1.35 (72³); 5 % of impurities 0.58 to 1.04.  So both are timed, as
+// the autotuner does.  Lattices that run several steps per launch are always faster by
+// patterns (0.64 to 0.91), and in FP64 the patterns never lose (0.43 to 1.01).
+void choose_words_or_patterns(asd_handle* h) {
+    configure_stage(h, 256, (int)STAGE_PATTERN);
+    if (!h->pat_varied || h->p.precision != ASD_FP32 || h->sell.stage != STAGE_PATTERN || several_steps_fit(h)) return;
+    // whole steps from the default spins, which set_default_spins puts back (the first stage alone picks
+    // wrongly by up to 5 %)
+    const uint64_t before = h->launches;
+    scatter_if_needed(h);
+    float best[2] = {1e30f, 1e30f};
+    for (int k = 0; k < 6; k++) {
+        constexpr int REPS = 4;
+        configure_stage(h, 256, k & 1 ? 1 : (int)STAGE_PATTERN);
+        CK(launch_fused_step(h, 0, false));
+        CK(cudaEventRecord(h->kev[0], h->stream));
+        for (int r = 0; r < REPS; r++) CK(launch_fused_step(h, 0, false));
+        CK(cudaEventRecord(h->kev[1], h->stream));
+        CK(cudaEventSynchronize(h->kev[1]));
+        float ms = 0.f;
+        CK(cudaEventElapsedTime(&ms, h->kev[0], h->kev[1]));
+        best[k & 1] = std::min(best[k & 1], ms / REPS);
+    }
+    h->launches = before;
+    for (int c = 0; c < 3; c++) CK(cudaMemsetAsync(h->detf[c], 0, sizeof(float) * h->n, h->stream));
+    set_default_spins(h);
+    const bool words = best[1] < best[0];
+    configure_stage(h, 256, words ? 1 : (int)STAGE_PATTERN);
+    char b[128];
+    std::snprintf(b, sizeof b, "block=%d staging=%s (timed: pattern %.4f, words %.4f ms per step)", h->block,
+                  words ? "words" : "pattern", (double)best[0], (double)best[1]);
+    h->tune = b;
 }
 
 // Project autotuner: time the first stage kind of the step (it writes only scratch buffers)
@@ -1245,12 +1299,7 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
         }
         // ---- default spins +z, then a graph for the fused forms
         uploads_done();
-        {
-            std::vector<double> s3(3 * (size_t)n, 0.0);
-            for (uint32_t i = 0; i < n; i++) s3[3 * (size_t)i + 2] = 1.0;
-            int rc = asd_set_spins(h, s3.data(), n);
-            if (rc != ASD_OK) throw Fail{rc, h->err};
-        }
+        set_default_spins(h);
         CK(cudaEventCreate(&h->kev[0]));
         CK(cudaEventCreate(&h->kev[1]));
         h->d_err = dalloc<uint32_t>(1);
@@ -1263,7 +1312,7 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
         CK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&h->d_lost), h->h_err + 1, 0));
         if (!plain) {
             if (p.flags & ASD_FLAG_AUTOTUNE) autotune(h);
-            else configure_stage(h, 256, (int)STAGE_PATTERN);
+            else choose_words_or_patterns(h);
             if (h->tune.empty()) {
                 static const char* names[4] = {"direct", "words", "words+spins", "pattern"};
                 char b[64];

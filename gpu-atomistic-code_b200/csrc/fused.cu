@@ -990,12 +990,15 @@ cudaError_t launch_fused_step(asd_handle* h, uint32_t rel, bool) {
     return fused_step_t<double>(h, rel);
 }
 
+bool several_steps_fit(const asd_handle* h) {
+    return h->pat.W && h->n <= (h->full ? RESIDENT_MAX_FULL : RESIDENT_MAX) && h->p.precision == ASD_FP32 &&
+           h->lr.mode == ASD_LR_NONE && !h->d_ttm && !h->sc.q4_ptr && step_pdl(h);
+}
+
 // Steps rel = 0 .. k-1 from the device step counter (phase h->step): one cooperative launch where the
 // lattice is small, its matrix has patterns and nothing else runs between the stages; else step by step.
 cudaError_t launch_fused_steps(asd_handle* h, uint32_t k) {
-    const bool one = k > 1 && h->n <= (h->full ? RESIDENT_MAX_FULL : RESIDENT_MAX) && h->p.precision == ASD_FP32 && h->dexch == ASD_EXCH_CSR &&
-                     h->sell.stage == STAGE_PATTERN && h->lr.mode == ASD_LR_NONE && !h->d_ttm && !h->sc.q4_ptr && step_pdl(h);
-    if (one) {
+    if (k > 1 && several_steps_fit(h) && h->dexch == ASD_EXCH_CSR && h->sell.stage == STAGE_PATTERN) {
         const bool comp = (h->p.flags & ASD_FLAG_COMPENSATED) != 0, heun = h->p.integrator == ASD_HEUN;
         ResidentArgs<float> ra = resident_args(h, comp);
         ra.nsteps = k;

@@ -194,6 +194,7 @@ struct asd_handle {
     double *detd[3] = {nullptr}, *stagd[3] = {nullptr};
     asd::SellDev sell;
     asd::PatDev pat;
+    bool pat_varied = false;             // many patterns (an alloy): patterns or words by timing
     asd::DiaDev dia;
     // FP64 plain (AoS [3i+c], reference-structured)
     double *p_s = nullptr, *p_es = nullptr, *p_fn = nullptr, *p_ch = nullptr, *p_hdemag = nullptr, *p_rand = nullptr,
@@ -285,6 +286,8 @@ namespace asd {
 cudaError_t launch_plain_step(asd_handle* h, uint64_t t);
 cudaError_t launch_fused_step(asd_handle* h, uint32_t rel, bool in_capture);
 cudaError_t launch_fused_steps(asd_handle* h, uint32_t k);
+// Whether several steps of this handle run as one launch when its stage kernels go by row patterns.
+bool several_steps_fit(const asd_handle* h);
 cudaError_t launch_step_advance(asd_handle* h, uint32_t nsteps);
 cudaError_t launch_det_here(asd_handle* h);
 // The one-step graph's det_here_k node with the applied field h->p.applied (no launch).

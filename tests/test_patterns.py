@@ -2,6 +2,8 @@
 (column - row, tensor)): bit-identical to the SELL gather of the same entries at ragged sizes,
 with boundary rows of every length, uneven replicas, full tensors and DIA input; a matrix whose
 rows do not repeat keeps its words."""
+import re
+
 import numpy as np
 import pytest
 
@@ -43,6 +45,35 @@ def test_patterns_bit_identical_to_sell(gpu, case, integ, prec):
         want, tune = run(s, prec, integ, shape)
         assert "pattern" not in tune, tune
         assert np.array_equal(got, want), shape
+
+
+def alloy(L, vecs, seed, nsp=2):
+    """Full pair tensors that go with the two sites' species: 2 to the power of (neighbours + 1) patterns."""
+    n = L[0] * L[1] * L[2]
+    J = np.array([1.0, 0.03, -0.03, -0.03, 1.0, 0.03, 0.03, -0.03, 1.0]) * 1e-21
+    xadj, adj, val = LT.build_csr(L, (1, 1, 1), [LT.MU_SC], [0] * len(vecs), [0] * len(vecs), vecs, [J] * len(vecs))
+    sp = np.random.default_rng(seed).integers(0, nsp, n)
+    rows = np.repeat(np.arange(n), np.diff(xadj))
+    val = np.ascontiguousarray(val.reshape(-1, 9) * (1.0 - 0.4 * sp[rows] - 0.3 * sp[adj])[:, None])
+    return A.SpinSystem(nspins=n, materials=[A.MaterialSpec(mu=LT.MU_SC, lam=0.1)], full=True, temperature=100.0,
+                        exch=A.EXCH_CSR, xadj=xadj, adjncy=adj, csr_val=val)
+
+
+def test_alloy_takes_the_faster_of_patterns_and_words(gpu):
+    """Many patterns: FP32 times both and keeps the faster; the results are the same.  FP64, and an alloy
+    that runs several steps per launch, go by patterns untimed."""
+    s = alloy((48, 48, 36), LT.SC_NNN, 3)
+    got, tune = run([s], A.FP32, A.HEUN)
+    m = re.search(r"staging=(\w+) \(timed: pattern ([\d.]+), words ([\d.]+)", tune)
+    assert m, tune
+    assert (m[1] == "words") == (float(m[3]) < float(m[2])) or m[2] == m[3], tune
+    want = run([s], A.FP32, A.HEUN, (64, 0))[0]
+    assert np.array_equal(got, want)
+    with A.Handle(A.RunParams(precision=A.FP32, flags=A.FLAG_COMPENSATED), s) as h:    # timing leaves no trace
+        assert h.t == 0 and not h.get_det_field().any()
+        assert np.array_equal(h.get_spins(), np.tile([0.0, 0.0, 1.0], (s.nspins, 1)))
+    assert "staging=pattern" in run([s], A.FP64_FUSED, A.HEUN)[1]
+    assert "staging=pattern (default)" in run([alloy((25, 25, 25), LT.SC_NN, 3)], A.FP32, A.HEUN)[1]
 
 
 def test_rows_that_do_not_repeat_keep_their_words(gpu):
