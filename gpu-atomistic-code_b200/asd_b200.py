@@ -458,7 +458,7 @@ class Handle:
         return raw.reshape(self._sq_nk, half), sm.reshape(self._sq_nk, half), pr, ps
 
     def tuning(self) -> str:
-        buf = C.create_string_buffer(512)
+        buf = C.create_string_buffer(1024)
         _check(load_library().asd_tuning(self.h, buf, len(buf)), self.h)
         return buf.value.decode()
 

@@ -1713,7 +1713,8 @@ int asd_tuning(const asd_handle* h, char* out, size_t out_len) {
     const char* lr = L.mode == ASD_LR_NONE ? "" : h->p.precision == ASD_FP64_PLAIN ? "; long-range: cuFFT Z2Z 3D"
                      : L.planes ? "; long-range: plane kernels" : L.pruned ? "; long-range: z-pass + cuFFT 2D planes"
                                                                        : "; long-range: cuFFT R2C/C2R 3D";
-    std::snprintf(out, out_len, "%s%s", h->tune.c_str(), lr);
+    const bool several = h->p.precision != ASD_FP64_PLAIN && several_steps(h);
+    std::snprintf(out, out_len, "%s%s%s", h->tune.c_str(), several ? "; steps: several per launch" : "", lr);
     return ASD_OK;
 }
 

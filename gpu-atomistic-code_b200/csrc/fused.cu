@@ -995,10 +995,14 @@ bool several_steps_fit(const asd_handle* h) {
            h->lr.mode == ASD_LR_NONE && !h->d_ttm && !h->sc.q4_ptr && step_pdl(h);
 }
 
+bool several_steps(const asd_handle* h) {
+    return several_steps_fit(h) && h->dexch == ASD_EXCH_CSR && h->sell.stage == STAGE_PATTERN;
+}
+
 // Steps rel = 0 .. k-1 from the device step counter (phase h->step): one cooperative launch where the
 // lattice is small, its matrix has patterns and nothing else runs between the stages; else step by step.
 cudaError_t launch_fused_steps(asd_handle* h, uint32_t k) {
-    if (k > 1 && several_steps_fit(h) && h->dexch == ASD_EXCH_CSR && h->sell.stage == STAGE_PATTERN) {
+    if (k > 1 && several_steps(h)) {
         const bool comp = (h->p.flags & ASD_FLAG_COMPENSATED) != 0, heun = h->p.integrator == ASD_HEUN;
         ResidentArgs<float> ra = resident_args(h, comp);
         ra.nsteps = k;

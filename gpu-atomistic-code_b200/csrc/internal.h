@@ -286,8 +286,10 @@ namespace asd {
 cudaError_t launch_plain_step(asd_handle* h, uint64_t t);
 cudaError_t launch_fused_step(asd_handle* h, uint32_t rel, bool in_capture);
 cudaError_t launch_fused_steps(asd_handle* h, uint32_t k);
-// Whether several steps of this handle run as one launch when its stage kernels go by row patterns.
+// Whether several steps of this handle would run as one launch if its stage kernels went by row
+// patterns, and whether they do.
 bool several_steps_fit(const asd_handle* h);
+bool several_steps(const asd_handle* h);
 cudaError_t launch_step_advance(asd_handle* h, uint32_t nsteps);
 cudaError_t launch_det_here(asd_handle* h);
 // The one-step graph's det_here_k node with the applied field h->p.applied (no launch).

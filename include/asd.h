@@ -319,8 +319,10 @@ int asd_kernel_stats(const asd_handle* h, char* name, size_t name_len, double* a
  * ASD_EINVAL when out_len is too small.  Measurement aid. */
 int asd_kernel_table(const asd_handle* h, char* out, size_t out_len);
 /* Launch shape of the fused stage kernel chosen at create (block size, shared-memory staging of
- * the typed exchange words), with ASD_FLAG_AUTOTUNE the autotuner's timings, and the transform
- * path of the long-range field. */
+ * the typed exchange words or row patterns), with ASD_FLAG_AUTOTUNE the autotuner's timings, whether
+ * asd_step of more than one step runs several steps per launch (small lattices; the block size is then
+ * that launch's own, and asd_time_kernels still times one launch per stage), and the transform path of
+ * the long-range field. */
 int asd_tuning(const asd_handle* h, char* out, size_t out_len);
 /* Set the fused stage kernel's launch shape by hand (by default a matrix whose rows repeat runs by
  * row patterns, which no staging mode selects): block in {64, 128, 256}; staging 1 stages
