@@ -754,7 +754,11 @@ void choose_words_or_patterns(asd_handle* h) {
 }
 
 // Project autotuner: time the first stage kind of the step (it writes only scratch buffers)
-// for every block size in {64, 128, 256} with and without staging, keep the fastest.
+// for every block size in {64, 128, 256} with and without staging, keep the fastest.  Where the row
+// patterns run several steps per launch, it is the fastest of the pattern shapes: one stage's launch
+// tells nothing of that (a small lattice's candidates differ by launch noise), and it wins throughout
+// (µs per step against the best of the other shapes: 210 spins 5.9 and 8.1, sc 16³ 5.8 and 8.3, 42³ 6.6
+// and 9.7; BCT-2 6×7×6 8.8 and 9.7, 21³ 9.2 and 10.9; RK4 the same way).
 void autotune(asd_handle* h) {
     struct Cand { uint32_t layout; int B; int mode; };
     static const char* names[4] = {"direct", "words", "words+spins", "pattern"};
@@ -784,6 +788,7 @@ void autotune(asd_handle* h) {
                       layouts.size() > 1 ? (cd.layout == ASD_EXCH_CSR ? "SELL:" : "DIA:") : "", cd.B, names[cd.mode],
                       (double)ms);
         log += buf;
+        if (several_steps_fit(h) && cd.mode != (int)STAGE_PATTERN) continue;
         if (ms < best) { best = ms; bc = cd; }
     }
     h->dexch = bc.layout;

@@ -71,6 +71,16 @@ def test_replicas_film_and_pulse(gpu):
     same([LT.film_dia(33, 21, 3, dipole=False)], integ=A.RK4, pulse=True)
 
 
+@pytest.mark.parametrize("s", [LT.sc_ferromagnet((7, 6, 5)), LT.sc_ferromagnet((16, 16, 8), pbc=(0, 0, 0)),
+                               LT.bct2_antiferromagnet((6, 7, 6))], ids=["sc7x6x5", "sc_open_dia", "bct2"])
+def test_autotuner_keeps_several_steps(gpu, s):
+    """One stage's launch time does not decide against the several-steps launch (launch noise did, on
+    two of three handles of the smallest lattice)."""
+    for _ in range(4):
+        with A.Handle(A.RunParams(precision=A.FP32, flags=A.FLAG_COMPENSATED | A.FLAG_AUTOTUNE), s) as h:
+            assert "staging=pattern; " in h.tuning() and "several per launch" in h.tuning(), h.tuning()
+
+
 def test_two_handles_at_once(gpu):
     """Two handles' streams hold such launches at the same time: each gets its own results."""
     s = LT.sc_ferromagnet((40, 40, 40), T=50.0)
