@@ -683,11 +683,15 @@ bool build_spin_stage(asd_handle* h, int B) {
     return true;
 }
 
+// Staging modes of the typed SELL words, by SellDev::stage.
+const char* const STAGE_NAMES[4] = {"direct", "words", "words+spins", "pattern"};
+
 // Launch shape of the fused stage kernel: block size and the staging mode of typed SELL
 // words (0 none, 1 words, 2 words and neighbour spins, STAGE_PATTERN row patterns instead of the
 // words where the matrix has them, else 1).
 void configure_stage(asd_handle* h, int B, int mode) {
     h->block = B;
+    h->stage_mode = mode;
     h->sell.stage = 0;
     h->sell.stage_words = 0;
     if (mode == 0 || !h->sell.typed || h->dexch != ASD_EXCH_CSR) return;
@@ -761,7 +765,6 @@ void choose_words_or_patterns(asd_handle* h) {
 // and 9.7; BCT-2 6×7×6 8.8 and 9.7, 21³ 9.2 and 10.9; RK4 the same way).
 void autotune(asd_handle* h) {
     struct Cand { uint32_t layout; int B; int mode; };
-    static const char* names[4] = {"direct", "words", "words+spins", "pattern"};
     std::vector<Cand> cs;
     // DIA input also exists as SELL-32, and a CSR matrix on few diagonals as DIA: both device
     // layouts are candidates
@@ -785,7 +788,7 @@ void autotune(asd_handle* h) {
         float ms = 0.f;
         CK(time_first_stage(h, 2, 8, &ms));
         std::snprintf(buf, sizeof buf, "%s%sB=%d/%s:%.4f", log.empty() ? "" : " ",
-                      layouts.size() > 1 ? (cd.layout == ASD_EXCH_CSR ? "SELL:" : "DIA:") : "", cd.B, names[cd.mode],
+                      layouts.size() > 1 ? (cd.layout == ASD_EXCH_CSR ? "SELL:" : "DIA:") : "", cd.B, STAGE_NAMES[cd.mode],
                       (double)ms);
         log += buf;
         if (several_steps_fit(h) && cd.mode != (int)STAGE_PATTERN) continue;
@@ -794,7 +797,7 @@ void autotune(asd_handle* h) {
     h->dexch = bc.layout;
     configure_stage(h, bc.B, bc.mode);
     std::snprintf(buf, sizeof buf, "%sblock=%d staging=%s; ", layouts.size() > 1 ? (bc.layout == ASD_EXCH_CSR ? "layout=SELL " : "layout=DIA ") : "",
-                  h->block, names[h->sell.stage]);
+                  h->block, STAGE_NAMES[h->sell.stage]);
     h->tune = std::string(buf) + "ms per stage launch: " + log;
 }
 
@@ -1319,9 +1322,8 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
             if (p.flags & ASD_FLAG_AUTOTUNE) autotune(h);
             else choose_words_or_patterns(h);
             if (h->tune.empty()) {
-                static const char* names[4] = {"direct", "words", "words+spins", "pattern"};
                 char b[64];
-                std::snprintf(b, sizeof b, "block=%d staging=%s (default)", h->block, names[h->sell.stage]);
+                std::snprintf(b, sizeof b, "block=%d staging=%s (default)", h->block, STAGE_NAMES[h->sell.stage]);
                 h->tune = b;
             }
             const uint32_t upd = p.update;
@@ -1607,9 +1609,8 @@ int asd_set_launch_shape(asd_handle* h, uint32_t block, uint32_t staging) {
         CK(cudaSetDevice(h->device));
         CK(cudaStreamSynchronize(h->stream));
         configure_stage(h, (int)block, (int)staging);
-        static const char* names[3] = {"direct", "words", "words+spins"};
         char b[64];
-        std::snprintf(b, sizeof b, "block=%d staging=%s (set)", h->block, names[h->sell.stage]);
+        std::snprintf(b, sizeof b, "block=%d staging=%s (set)", h->block, STAGE_NAMES[h->sell.stage]);
         h->tune = b;
         if (h->graph_steps) build_graph(h, h->graph_steps);
     } catch (const Fail& f) { return fail(h, f); }
@@ -1627,8 +1628,11 @@ int asd_set_device_layout(asd_handle* h, uint32_t layout) {
         CK(cudaSetDevice(h->device));
         CK(cudaStreamSynchronize(h->stream));
         h->dexch = layout;
-        configure_stage(h, h->block, h->sell.stage);
-        h->tune = std::string(layout == ASD_EXCH_CSR ? "layout=SELL " : "layout=DIA ") + h->tune;
+        configure_stage(h, h->block, h->stage_mode);
+        char b[80];
+        std::snprintf(b, sizeof b, "layout=%s block=%d staging=%s (set)", layout == ASD_EXCH_CSR ? "SELL" : "DIA",
+                      h->block, STAGE_NAMES[h->sell.stage]);
+        h->tune = b;
         if (h->graph_steps) build_graph(h, h->graph_steps);
     } catch (const Fail& f) { return fail(h, f); }
     return ASD_OK;

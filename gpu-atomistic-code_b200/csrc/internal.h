@@ -194,6 +194,7 @@ struct asd_handle {
     double *detd[3] = {nullptr}, *stagd[3] = {nullptr};
     asd::SellDev sell;
     asd::PatDev pat;
+    int stage_mode = 0;                  // staging mode asked for (SellDev::stage: the one in force)
     bool pat_varied = false;             // many patterns (an alloy): patterns or words by timing
     asd::DiaDev dia;
     // FP64 plain (AoS [3i+c], reference-structured)

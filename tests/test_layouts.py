@@ -50,6 +50,18 @@ def test_matrix_on_many_diagonals_has_no_dia_layout(gpu):
             h.set_device_layout(A.EXCH_DIA)
 
 
+def test_staging_survives_a_change_of_layout(gpu):
+    """DIA stages nothing; back on SELL the handle stages as before, by default by row patterns."""
+    s = LT.sc_ferromagnet((16, 16, 8), pbc=(0, 0, 0))
+    for shape, name in ((None, "pattern"), ((128, 1), "words"), ((64, 0), "direct")):
+        with A.Handle(A.RunParams(precision=A.FP32, flags=A.FLAG_COMPENSATED), s) as h:
+            if shape:
+                h.set_launch_shape(*shape)
+            for layout, want in ((A.EXCH_DIA, "direct"), (A.EXCH_CSR, name), (A.EXCH_CSR, name)):
+                h.set_device_layout(layout)
+                assert f"staging={want} " in h.tuning(), h.tuning()
+
+
 def test_autotuner_considers_both_layouts(gpu):
     s = LT.sc_ferromagnet((16, 16, 8), pbc=(0, 0, 0))
     with A.Handle(A.RunParams(precision=A.FP32, flags=A.FLAG_COMPENSATED | A.FLAG_AUTOTUNE), s) as h:
