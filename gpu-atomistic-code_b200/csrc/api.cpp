@@ -473,34 +473,12 @@ void setup_lr(asd_handle* h, const asd_system& s, bool plain) {
         const uint32_t m = L.mesh[a];
         if (m % 2 == 0 && h->n > 0 && hi[a] - lo[a] < m / 2) clear |= 1u << a;
     }
-    // The plane kernels where their axis lengths, the box and the shared memory fit; a complex N_k
-    // must fit as well unless N_r is even over the box (then N_k is real).
+    // The plane kernels where their axis lengths, the box and the shared memory fit.
     const uint32_t box[3] = {hi[0] - lo[0] + 1, hi[1] - lo[1] + 1, hi[2] - lo[2] + 1};
-    auto even = [&]() {
-        if (!sym) return false;
-        for (uint32_t x = 0; x < box[0]; x++)
-            for (uint32_t y = 0; y < 2 * box[1] - 1; y++)
-                for (uint32_t z = 0; z < 2 * box[2] - 1; z++) {
-                    const uint32_t dy = y < box[1] ? y : s.mesh[1] - (y - box[1] + 1);
-                    const uint32_t dz = z < box[2] ? z : s.mesh[2] - (z - box[2] + 1);
-                    const uint32_t c[3] = {x, dy, dz};
-                    size_t at = 0, mir = 0;
-                    for (int a = 0; a < 3; a++) {
-                        at = at * s.mesh[a] + c[a];
-                        mir = mir * s.mesh[a] + (c[a] ? s.mesh[a] - c[a] : 0);
-                    }
-                    for (int q = 0; q < 9; q++)
-                        if (std::fabs(s.nr[q * L.P + at] - s.nr[q * L.P + mir]) > 1e-13 * amax) return false;
-                }
-        return true;
-    };
-    auto fits = [&](const LongRange& l) {
-        return plane_path_fits(l, false) && (plane_path_fits(l, true) || even());
-    };
-    uint32_t org[3] = {0, 0, 0};                       // mesh position of the caller's origin, negated
+    uint32_t org[3] = {0, 0, 0};                       // the caller's mesh point that becomes the origin
     if (!plain && h->n > 0 && !(h->p.flags & ASD_FLAG_CUFFT_PLANES)) {
         for (int a = 0; a < 3; a++) { L.box0[a] = lo[a]; L.box1[a] = hi[a]; }
-        L.planes = fits(L) ? 1 : 0;
+        L.planes = plane_path_fits(L) ? 1 : 0;
         // Another mesh: where no two spins of the box alias on the caller's mesh, its N_r holds
         // every interaction at one displacement each, and the convolution is the same on any mesh
         // of at least twice the box.  A mesh whose axes are not lengths of the plane kernels
@@ -518,7 +496,7 @@ void setup_lr(asd_handle* h, const asd_system& s, bool plain) {
             LongRange t = L;
             plane_mesh_for(box, t.mesh);
             for (int a = 0; a < 3; a++) { t.box0[a] = 0; t.box1[a] = box[a] - 1; }
-            if (t.mesh[0] && t.mesh[1] && t.mesh[2] && fits(t)) {
+            if (t.mesh[0] && t.mesh[1] && t.mesh[2] && plane_path_fits(t)) {
                 L = t;
                 L.planes = 1;
                 L.P = (size_t)L.mesh[0] * L.mesh[1] * L.mesh[2];

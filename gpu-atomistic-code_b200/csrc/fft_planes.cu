@@ -905,7 +905,8 @@ cudaError_t run_xconv(const LongRange& L, const PlaneArgs& A, bool cplx, cudaStr
 }  // namespace
 
 // Axis lengths of the plane kernels' transforms, ascending: powers of two and 3 x powers of two
-// (from 48 on, where the step from one power of two to the next costs time).
+// (24 along x; from 48 on along every axis, where the step from one power of two to the next costs
+// time).
 constexpr uint32_t X_LEN[] = {4, 8, 16, 24, 32, 48, 64, 96, 128, 192, 256};
 constexpr uint32_t Y_LEN[] = {8, 16, 32, 48, 64, 96, 128, 192, 256};
 constexpr uint32_t Z_LEN[] = {8, 16, 32, 48, 64, 96, 128, 192, 256, 512};
@@ -922,14 +923,13 @@ uint32_t len_from(const uint32_t (&len)[K], uint32_t least) {
 // spans at most half the mesh along x and y and its z pairs fit in half a row (so every forward
 // pass skips the zero half of its input and every inverse pass forms only the box half of its
 // output), and the shared memory fits.
-bool plane_path_fits(const LongRange& L, bool cplx) {
+bool plane_path_fits(const LongRange& L) {
     if (!has_len(X_LEN, L.mesh[0]) || !has_len(Y_LEN, L.mesh[1]) || !has_len(Z_LEN, L.mesh[2])) return false;
-    LongRange t = L;
-    t.nk_nkx = L.mesh[0];                              // the larger N_k tile bounds the shared memory
-    const PlaneArgs A = plane_args(t);
+    const PlaneArgs A = plane_args(L);
     const uint32_t N = L.mesh[2] / 2;
     if (2 * A.bx > L.mesh[0] || 2 * A.by > L.mesh[1] || 2 * A.nz > N) return false;
-    return zy_smem(L, A) <= 200 * 1024 && xconv_smem(A, cplx) <= 220 * 1024;
+    // (the complex N_k's tile is the larger; over all lengths it takes at most 191,488 bytes)
+    return zy_smem(L, A) <= 200 * 1024 && xconv_smem(A, true) <= 220 * 1024;
 }
 
 // The shortest mesh of the plane kernels that holds twice the box (0 in an axis: none does).

@@ -305,7 +305,7 @@ cudaError_t run_zy_part1(const LongRange& L, bool inverse, cudaStream_t st, bool
 cudaError_t run_zy_part2(const LongRange& L, bool inverse, cudaStream_t st, bool pdl);
 cudaError_t run_zy_part3(const LongRange& L, bool inverse, cudaStream_t st, bool pdl);
 cudaError_t build_plane_twiddles(asd_handle* h);
-bool plane_path_fits(const LongRange& L, bool cplx);
+bool plane_path_fits(const LongRange& L);
 void plane_mesh_for(const uint32_t box[3], uint32_t mesh[3]);
 // The caller's N_r on the device: the m/2 planes of the axes in `clear` zeroed, and the (a,b), (b,a)
 // pairs of a symmetric matrix replaced by their mean.
