@@ -488,15 +488,23 @@ void setup_lr(asd_handle* h, const asd_system& s, bool plain) {
         // 90×75×41 (180×150×82 → 192×192×96) 207.9 → 69.7, 100×100×60 274.8 → 132.1, 30³ 33.0 →
         // 19.9, 20×25×9 25.5 → 17.8, 120×100×3 37.9 → 33.6.  A power-of-two mesh of 2 or 4 z points
         // (films of one or two layers) stays: the plane kernels' shortest z axis is 8, and cuFFT's
-        // power-of-two planes win (128×128×1 31.3 against 34.3).
+        // power-of-two planes win (128×128×1 31.3 against 34.3).  Other films of one and two layers move
+        // (65×65×1 40.2 → 26.4, 127×127×2 100.6 → 34.6, 50×50×1 24.3 → 22.4; where x goes to 256 from a
+        // length of small factors within 8 % either way: 120×120×1 36.2 → 33.2, 108×108×2 30.9 → 33.1,
+        // 100×100×1 32.6 → 31.5).  A chain along x of such a length (200 to 250) stays: the transform is
+        // all latency there (100×1×1 22.2 against 23.4, 125×1×1 21.6 against 23.7; 97×1×1, with a factor
+        // 97, moves: 28.8 → 22.7).
         const bool p2 = !((L.mesh[0] & (L.mesh[0] - 1)) | (L.mesh[1] & (L.mesh[1] - 1)) | (L.mesh[2] & (L.mesh[2] - 1)));
         bool alone = true;
         for (int a = 0; a < 3; a++) alone &= 2 * box[a] <= L.mesh[a] + 1;
         if (!L.planes && alone && !(p2 && L.mesh[2] <= 4)) {
             LongRange t = L;
             plane_mesh_for(box, t.mesh);
+            uint32_t rest = L.mesh[0];
+            for (uint32_t f : {2u, 3u, 5u}) while (rest % f == 0) rest /= f;
+            const bool short_chain = box[1] == 1 && box[2] == 1 && t.mesh[0] == 256 && rest == 1;
             for (int a = 0; a < 3; a++) { t.box0[a] = 0; t.box1[a] = box[a] - 1; }
-            if (t.mesh[0] && t.mesh[1] && t.mesh[2] && plane_path_fits(t)) {
+            if (t.mesh[0] && t.mesh[1] && t.mesh[2] && !short_chain && plane_path_fits(t)) {
                 L = t;
                 L.planes = 1;
                 L.P = (size_t)L.mesh[0] * L.mesh[1] * L.mesh[2];

@@ -19,14 +19,14 @@ FP32 = (A.FP32, A.FLAG_COMPENSATED, 1e-5)
 FUSED64 = (A.FP64_FUSED, 0, 1e-8)
 
 
-def check(s, steps, forms=(FP32, FUSED64)):
+def check(s, steps, forms=(FP32, FUSED64), path=PLANES):
     S0 = LT.random_spins(s.nspins, 0)
     o = O.Oracle(s)
     o.set_spins(S0)
     o.step(steps)
     for prec, flags, tol in forms:
         with A.Handle(A.RunParams(precision=prec, flags=flags), s) as h:
-            assert PLANES in h.tuning(), h.tuning()
+            assert path in h.tuning(), h.tuning()
             h.set_spins(S0)
             h.step(steps)
             g = h.get_spins()
@@ -45,6 +45,12 @@ def check(s, steps, forms=(FP32, FUSED64)):
                                (87, 9, 3)])      # 192, 32, 8
 def test_ragged_dipole_matches_oracle(gpu, L):
     check(LT.sc_ferromagnet(L, pbc=(0, 0, 0), dipole=True), 10)
+
+
+@pytest.mark.parametrize("L, path", [(125, "cuFFT"), (97, PLANES), (96, PLANES), (128, "cuFFT")])
+def test_chain(gpu, L, path):
+    """A chain along x stays on cuFFT where its mesh length has small factors and would go to 256."""
+    check(LT.sc_ferromagnet((L, 1, 1), pbc=(0, 0, 0), dipole=True), 20, path=path)
 
 
 def test_ragged_box_away_from_origin(gpu):
