@@ -1,4 +1,4 @@
-// Device building blocks of the long-range-field transforms (FP32, power-of-two sizes).
+// Device building blocks of the long-range-field transforms (FP32; powers of two, and 24, 48, 96, 192).
 //
 //  * dft<R, INV>: R-point DFT (R = 2, 3, 4, 6, 8, 12, 16) of a register array, natural
 //    order in and out, from radix 4, 2 and 3 with compile-time twiddles (multiplications by +-1,
@@ -34,10 +34,12 @@ __device__ __forceinline__ float2 tw16(float2 a, int e) {
     constexpr float C1 = 0.92387953251128676f;   // cos(pi/8)
     constexpr float S1 = 0.38268343236508977f;   // sin(pi/8)
     constexpr float H = 0.70710678118654752f;    // sqrt(1/2)
-    // C1 and H round down: with them alone a convolution (three axes, there and back) comes out 9e-8
-    // too small on average, the same at every step.  Half of the C1 twiddles and the real part of
-    // w_16^6 take the next float above, which leaves less than 1e-8 (mean gain of the passes on a box of
-    // half the axis, per axis there and back: 64 points -2.0e-8 → -0.1e-8, 256 -2.9e-8 → 0.2e-8).
+    // C1 and H round down: with every constant and the twiddle table rounded to nearest the field of
+    // random spins comes out 1.2e-7 too small (64³ mesh; 1.5e-7 on 256×256×64), the same at every step.
+    // Half of the C1 twiddles and the real part of w_16^6 take the next float above, which with the
+    // table's own choice leaves -1.4e-8 (0.3e-8), and an rms error of 1.26e-7 instead of 1.67e-7 (1.40e-7
+    // instead of 1.97e-7).  Per axis there and back (trace over the box): 64 points -3.8e-8 → -0.5e-8, 256
+    // -5.3e-8 → 0.5e-8.
     constexpr float C1U = 0.92387956380844116f, HU = 0.70710682868957520f;
     const float sg = INV ? 1.0f : -1.0f;         // sign of the imaginary part of w_16^1
     switch (e & 15) {
@@ -138,9 +140,12 @@ struct Dft<4, INV> {
 template <bool INV>
 struct Dft<3, INV> {
     static __device__ __forceinline__ void run(float2* v) {
-        // sin(2 pi / 3) rounded up, against the other constants' rounding down (tw16): mean gain of
-        // 48 points -1.5e-8 → 0.0e-8, 192 points -1.3e-8 → 0.4e-8
-        constexpr float S3 = 0.86602544784545898f;
+        // sin(2 pi / 3): forward the nearest float, which is below it, inverse the next above.  Common
+        // factor of one axis there and back (trace over the box), both nearest / both above / as here:
+        // 48 points -2.4e-8 / 2.2e-8 / -0.1e-8, 96 -1.5e-8 / 3.0e-8 / 0.8e-8, 192 -2.2e-8 / 2.4e-8 / 0.1e-8.
+        // Field of random spins on a 48³ mesh, both above → as here: 6.8e-8 → 0.1e-8, rms error 1.48e-7 →
+        // 1.25e-7; on 192×192×96 5.4e-8 → -1.5e-8, 1.41e-7 → 1.26e-7.
+        constexpr float S3 = INV ? 0.86602544784545898f : 0.86602538824081421f;
         const float2 t = cadd(v[1], v[2]), d = csub(v[1], v[2]);
         const float2 m = make_float2(v[0].x - 0.5f * t.x, v[0].y - 0.5f * t.y);
         const float2 s = mul_mi<INV>(make_float2(S3 * d.x, S3 * d.y));
