@@ -514,8 +514,10 @@ def test_dependent_launch_bit_identical(gpu, prec):
     while its predecessor finishes, and wait for it before touching memory) against strictly
     ordered launches (ASD_FLAG_SERIAL_LAUNCH), through the 32-step graphs, the one-step graph
     and direct launches: bit-identical spins at finite temperature, with the plane-kernel dipole
-    field and with RK4."""
+    field and with RK4.  (In FP32 the smallest lattice's chunks are one launch of several steps; the
+    next is the first size past that.)"""
     cases = [(LT.bct2_antiferromagnet(5, T=300.0), {}),
+             (LT.sc_ferromagnet((148, 19, 27), T=100.0), {}),
              (LT.sc_ferromagnet((16, 16, 8), pbc=(0, 0, 0), dipole=True, T=100.0), {}),
              (LT.film_dia(12, 10, 3, dipole=True), dict(integrator=A.RK4))]
     for s, kw in cases:

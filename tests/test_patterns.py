@@ -1,7 +1,9 @@
 """The stage kernels' row patterns (each row a 2-byte number into the distinct sequences of
 (column - row, tensor)): bit-identical to the SELL gather of the same entries at ragged sizes,
 with boundary rows of every length, uneven replicas, full tensors and DIA input; a matrix whose
-rows do not repeat keeps its words."""
+rows do not repeat keeps its words.  Single steps run the stage kernels, which whole chunks of these
+small lattices in FP32 do not (tests/test_resident_steps.py); the kernels that only larger lattices
+take are run at the sizes where each begins."""
 import re
 
 import numpy as np
@@ -23,14 +25,15 @@ CASES = {
 }
 
 
-def run(systems, prec, integ, shape=None):
+def run(systems, prec, integ, shape=None, steps=40, single=False):
     flags = A.FLAG_COMPENSATED if prec == A.FP32 else 0
     n = sum(s.nspins for s in systems)
     with A.Handle(A.RunParams(precision=prec, flags=flags, integrator=integ, seed=4), systems) as h:
         if shape:
             h.set_launch_shape(*shape)
         h.set_spins(LT.random_spins(n, 5))
-        h.step(40)
+        for k in [1] * steps if single else [steps]:
+            h.step(k)
         return h.get_spins(), h.tuning()
 
 
@@ -41,10 +44,28 @@ def test_patterns_bit_identical_to_sell(gpu, case, integ, prec):
     s = CASES[case]()
     got, tune = run(s, prec, integ)
     assert "staging=pattern" in tune, tune
+    assert np.array_equal(got, run(s, prec, integ, single=True)[0])
     for shape in ((256, 1), (64, 0)):
         want, tune = run(s, prec, integ, shape)
         assert "pattern" not in tune, tune
         assert np.array_equal(got, want), shape
+
+
+# FP32, one wave of 4 blocks of 256 per SM being 151,552 rows: the last size of the early-loading
+# kernels and the first past it, diagonal tensors of 6 neighbours (48 registers past one wave) and of
+# 18 (64 up to two waves, then 48), and full tensors (64)
+@pytest.mark.parametrize("integ", [A.HEUN, A.RK4])
+@pytest.mark.parametrize("make", [lambda: LT.sc_ferromagnet((148, 32, 32), T=100.0),
+                                  lambda: LT.sc_ferromagnet((148, 32, 33), T=100.0),
+                                  lambda: LT.film_dia(148, 74, 14, dipole=False),
+                                  lambda: LT.film_dia(148, 74, 28, dipole=False),
+                                  lambda: LT.bct2_antiferromagnet((37, 64, 33), T=100.0)],
+                         ids=["one_wave", "diag6", "diag18_two_waves", "diag18", "full"])
+def test_large_lattice_kernels_bit_identical_to_sell(gpu, make, integ):
+    s = make()
+    got, tune = run([s], A.FP32, integ, steps=6)
+    assert "staging=pattern" in tune and "several" not in tune, tune
+    assert np.array_equal(got, run([s], A.FP32, integ, (256, 1), steps=6)[0])
 
 
 def alloy(L, vecs, seed, nsp=2):
