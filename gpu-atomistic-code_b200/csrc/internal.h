@@ -62,7 +62,7 @@ struct PatDev {
 constexpr int32_t PAT_DELTA = 1 << 23;  // |column - row| is below this
 constexpr uint32_t STAGE_PATTERN = 3;   // SellDev::stage: the stage kernels gather by row patterns
 // the stage kernel's layout parameter in that mode: at 48 registers, at 64 (see MinBlocks), and at
-// 64 with the first neighbours loaded early (see stage_kernel)
+// 64 with the first neighbours loaded early (see pattern_kernel)
 constexpr int EXCH_PATTERN = 4, EXCH_PATTERN_64 = 5, EXCH_PATTERN_EARLY = 6;
 constexpr uint32_t MAG_CHUNK = 2048;  // spins per block of the magnetisation reduction
 constexpr uint32_t SPIN_PAD = 8;     // zeroed elements after every gather-source spin array
@@ -115,7 +115,7 @@ struct LongRange {
     float2* k1 = nullptr;
     float2* k2 = nullptr;
     cufftHandle c2c = 0;
-    // plane path (every axis a power of two, x and y <= 256): the library's own three kernels
+    // plane path (every axis a power of two or 3 x one, x and y <= 256, z <= 512): the library's own three kernels
     // (z+y forward, x + N_k product + inverse x, inverse y+z); the spectrum yk is
     // [c][kz][ky tile][box x][8] and N_k is tiled to match ([kz][tile][comp][kx][8])
     int planes = 0;
