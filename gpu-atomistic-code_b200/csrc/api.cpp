@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -1325,6 +1326,11 @@ int asd_create(const asd_params* pp, const asd_system* sys, uint32_t nsys, asd_h
         free_all(h);
         delete h;
         return code;
+    } catch (const std::bad_alloc&) {    // the host copies of a large matrix
+        g_create_err = "out of host memory";
+        free_all(h);
+        delete h;
+        return ASD_ENOMEM;
     }
     *out = h;
     return ASD_OK;
