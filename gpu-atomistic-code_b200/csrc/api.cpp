@@ -735,6 +735,8 @@ void choose_words_or_patterns(asd_handle* h) {
     }
     h->launches = before;
     for (int c = 0; c < 3; c++) CK(cudaMemsetAsync(h->detf[c], 0, sizeof(float) * h->n, h->stream));
+    if (h->lr.mode != ASD_LR_NONE)
+        CK(cudaMemsetAsync(h->lr.r + 3 * h->lr.P, 0, sizeof(float) * 3 * h->lr.P, h->stream));
     set_default_spins(h);
     const bool words = best[1] < best[0];
     configure_stage(h, 256, words ? 1 : (int)STAGE_PATTERN);

@@ -93,6 +93,13 @@ def test_alloy_takes_the_faster_of_patterns_and_words(gpu):
     with A.Handle(A.RunParams(precision=A.FP32, flags=A.FLAG_COMPENSATED), s) as h:    # timing leaves no trace
         assert h.t == 0 and not h.get_det_field().any()
         assert np.array_equal(h.get_spins(), np.tile([0.0, 0.0, 1.0], (s.nspins, 1)))
+        f = h.get_field()
+    s.nr, s.mesh = LT.dipole_nr((48, 48, 36))
+    s.lr, s.mesh_xyz = A.LR_DIPOLE, LT.sc_mesh_xyz((48, 48, 36))
+    with A.Handle(A.RunParams(precision=A.FP32, flags=A.FLAG_COMPENSATED), s) as h:    # nor in the dipole field
+        assert "timed:" in h.tuning(), h.tuning()
+        assert np.array_equal(h.get_field(), f)
+    s.lr = A.LR_NONE
     assert "staging=pattern" in run([s], A.FP64_FUSED, A.HEUN)[1]
     assert "staging=pattern (default)" in run([alloy((25, 25, 25), LT.SC_NN, 3)], A.FP32, A.HEUN)[1]
 
